@@ -195,7 +195,7 @@ struct GatedAct {
   int kind;
   float beta;
   float linear_beta;
-  const uint16_t* silu_tab;   // optional: bf16 bits of silu(g) for every bf16 g (65536 entries), or nullptr
+  int direct;                 // SiLU: evaluate the expression itself (testing) instead of its short form
 };
 
 static __device__ __noinline__ float situ_act(float g, float u, float beta, float linear_beta) {
@@ -211,27 +211,60 @@ __device__ __forceinline__ float silu_direct(float g) {
   float s = __fdiv_rn(g, __fadd_rn(1.0f, expf(-g)));
   return __bfloat162float(__float2bfloat16_rn(s));
 }
-// The same through the table: the gate has only 65536 possible values, and the table is filled with
-// silu_direct on the device, so both give the same bits.  One cached load replaces expf, an IEEE
-// division (whose slow-path branch also keeps the compiler from interleaving neighbouring
-// elements) and a rounding.
-__device__ __forceinline__ float silu_lookup(float g, const uint16_t* tab) {
-  return __uint_as_float((uint32_t)__ldg(tab + (__float_as_uint(g) >> 16)) << 16);
-}
-__device__ __forceinline__ float silu_mul(float g, float u, const uint16_t* tab) {
-  return __bfloat162float(__float2bfloat16_rn(__fmul_rn(silu_lookup(g, tab), u)));
+// The same bits in a handful of instructions: the approximate exponential and reciprocal are good to a few units in the
+// last place of a float, and for none of the 65536 bf16 gates does that move the result across a bf16 rounding boundary
+// (checked for every pattern by the tests).  The direct form's expf and IEEE division cost about 40 instructions with a
+// slow-path branch; a 65536-entry table in global memory cost one gathered load per gate, which the L1 serves at about
+// 14 cycles per warp - that, not memory, was the bound of both users (gated quantizer 57 us for 12000 x 2880 outputs).
+__device__ __forceinline__ float silu_short(float g) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmul_rn(g, -1.44269504088896341f)));      // exp(-g)
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(__fadd_rn(1.0f, e)));
+  return __fmul_rn(g, r);
 }
 
-// General form (any activation kind, with or without the table).  SiLU is the hot case and stays
-// inline; SiTU is a call, so a caller's unrolled loop stays small.
+// General form (any activation kind).  SiLU is the hot case and stays inline; SiTU is a call, so a caller's unrolled
+// loop stays small.
 __device__ __forceinline__ float gated_act(float g, float u, const GatedAct& a) {
   if (a.kind == PNV_ACT_SITU) return situ_act(g, u, a.beta, a.linear_beta);
-  float s_bf = a.silu_tab != nullptr ? silu_lookup(g, a.silu_tab) : silu_direct(g);
+  const float s_bf = a.direct ? silu_direct(g) : __bfloat162float(__float2bfloat16_rn(silu_short(g)));
   return __bfloat162float(__float2bfloat16_rn(__fmul_rn(s_bf, u)));
 }
 
-// (activation kind, beta, linear_beta) -> GatedAct with the reference's argument checks; for SiLU it also
-// makes sure the lookup table of the current device is filled before anything later on `stream` runs (quant.cu)
-int make_gated_act(int act_kind, float beta, float linear_beta, cudaStream_t stream, GatedAct& out);
+// ---- two bf16 to a register ----------------------------------------------------------------------
+__device__ __forceinline__ __nv_bfloat162 as_bf162(uint32_t w) { return *reinterpret_cast<const __nv_bfloat162*>(&w); }
+__device__ __forceinline__ uint32_t as_u32(__nv_bfloat162 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+// Element-wise max of two pairs of magnitudes (a NaN loses to a number, as with fmaxf).
+__device__ __forceinline__ uint32_t bf16x2_max(uint32_t a, uint32_t b) { return as_u32(__hmax2(as_bf162(a), as_bf162(b))); }
+// Largest magnitude of eight pairs, separately for the low and the high halves.
+__device__ __forceinline__ uint32_t bf16x2_amax8(const uint32_t (&y)[8]) {
+  uint32_t m = y[0] & 0x7FFF7FFFu;
+#pragma unroll
+  for (int i = 1; i < 8; ++i) m = bf16x2_max(m, y[i] & 0x7FFF7FFFu);
+  return m;
+}
+// quant8 for values that sit in four such registers.
+__device__ __forceinline__ uint32_t quant8_packed(uint32_t a, uint32_t b, uint32_t c, uint32_t d, float inv) {
+  const float f[8] = {bf16_lo(a), bf16_hi(a), bf16_lo(b), bf16_hi(b), bf16_lo(c), bf16_hi(c), bf16_lo(d), bf16_hi(d)};
+  return quant8(f, inv);
+}
+// The gated activation of 16 neighbouring features.  silu(g) is a bf16 number and the product of two bf16 numbers is
+// exact in float, so one packed bf16 multiplication rounds like the float product rounded to bf16.
+__device__ __forceinline__ void gated_act16(const uint32_t (&g)[8], const uint32_t (&u)[8], const GatedAct& a, uint32_t (&y)[8]) {
+  if (a.kind == PNV_ACT_SILU && !a.direct) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const __nv_bfloat162 s = __floats2bfloat162_rn(silu_short(bf16_lo(g[i])), silu_short(bf16_hi(g[i])));
+      y[i] = as_u32(__hmul2(s, as_bf162(u[i])));
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      y[i] = as_u32(__floats2bfloat162_rn(gated_act(bf16_lo(g[i]), bf16_lo(u[i]), a), gated_act(bf16_hi(g[i]), bf16_hi(u[i]), a)));
+  }
+}
+
+// (activation kind, beta, linear_beta) -> GatedAct with the reference's argument checks (quant.cu)
+int make_gated_act(int act_kind, float beta, float linear_beta, GatedAct& out);
 
 }  // namespace pnv

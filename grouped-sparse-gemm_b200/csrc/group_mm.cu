@@ -124,7 +124,7 @@ struct Params {
   int sfb_rt;        // scale row-atoms per expert in sfb = ceil(max_n / 128)
   int stages;        // pipeline depth in use (<= Cfg::kStages)
   int b_4d;          // map_b is the 4-D view [E][K/256][max_n][128 B] and one copy fetches a whole stage
-  int prod_lanes;    // wide kernel: lanes of each producer warp that issue copies side by side
+  int out_tma;       // wide kernel, plain epilogue: map_out describes `out` and whole chunks leave through it
   int b_tail;        // wide kernel: a second activation map with a 64-token box exists (narrow tail tiles)
   // narrow kernel, split K (nullptr = every tile on one CTA): per-tile arrival counters (all zero before and
   // after a launch) followed by two partial-accumulator slots per CTA
@@ -584,11 +584,6 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           for (int i = 0; i < kCols; ++i) buf[i * kOutRow + m_local] = h[i];
           epilogue_bar_sync();
           constexpr int kHalf = kCols / 2;
-          // decode-sized tiles have few pairs per lane: evaluate SiLU directly rather than through the
-          // table, whose loads (global memory, mostly L2 with this kernel's shared-memory carve-out) only
-          // add latency here
-          GatedAct act = p.f_act;
-          act.silu_tab = nullptr;
           const int par = is_up ? 1 : 0;
           const int g_row = is_up ? m_local - 32 : m_local;   // the gate's slot, which receives the product
           __nv_bfloat16* col0 = buf + par * kOutRow + g_row;
@@ -602,7 +597,7 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             }
             __nv_bfloat16 y[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) y[i] = __float2bfloat16_rn(gated_act(g[i], u[i], act));
+            for (int i = 0; i < 4; ++i) y[i] = __float2bfloat16_rn(gated_act(g[i], u[i], p.f_act));
 #pragma unroll
             for (int i = 0; i < 4; ++i) col0[(i0 + i) * 2 * kOutRow] = y[i];
           }
@@ -779,6 +774,25 @@ int make_map(CUtensorMap* map, const void* base, uint64_t row_bytes, uint64_t ro
   });
 }
 
+// The bf16 output [experts][rows][features] in boxes of 64 features x box_rows rows (128-byte swizzle).
+int make_map_out(CUtensorMap* map, const void* base, uint64_t features, uint64_t rows, uint64_t experts, uint32_t box_rows) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return fail(PNV_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  return cached_map(map, MapKey{base, features * 2, rows, experts, box_rows, 64, 2u}, [&](CUtensorMap* m) {
+    cuuint64_t dims[3] = {features, rows, experts};
+    cuuint64_t strides[2] = {features * 2, features * 2 * rows};
+    cuuint32_t box[3] = {64, box_rows, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS)
+      return fail(PNV_ERR_CUDA, "cuTensorMapEncodeTiled (output) failed with CUresult %d (features=%llu rows=%llu)", (int)r,
+                  (unsigned long long)features, (unsigned long long)rows);
+    return (int)PNV_OK;
+  });
+}
+
 // Per kernel instantiation and device, once: opt in to the large dynamic shared-memory carve-out and
 // (CTA pairs) allow the cluster launch and ask how many pairs the device runs at the same time.
 struct KernelSetup {
@@ -848,8 +862,8 @@ int launch_narrow(const CUtensorMap& map_a, const CUtensorMap& map_b, Params& p,
 // Pipeline depth of a wide-tile launch: what fits beside the epilogue staging, the barriers and the
 // counts, capped by the scale-slot ring in tensor memory.
 template <class C>
-int wide_stages(int experts, bool fused) {
-  const int fixed = 1024 + (fused ? C::kFusedOutBytes : C::kPlainOutBytes) + C::kBarrierBytes + 4 * experts;
+int wide_stages(int experts) {
+  const int fixed = 1024 + C::kOutBytes + C::kBarrierBytes + 8 * experts;
   int n = std::min(std::min((int)C::kMaxStages, (int)C::kSlots), (kSmemLimit - fixed) / C::kStageBytes);
 #ifdef PNV_WIDE_MAX_STAGES      // developer builds: a shallower ring, to see how the time depends on its depth
   n = std::min(n, PNV_WIDE_MAX_STAGES);
@@ -858,17 +872,17 @@ int wide_stages(int experts, bool fused) {
 }
 
 template <int TILE_N, int STAGE_K, bool kFused, bool kPair, bool kDblTails = false>
-int launch_wide_impl(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_b_tail, const Params& p_in,
+int launch_wide_impl(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_b_tail, const CUtensorMap& map_out,
+                     const Params& p_in,
                      int sm_count, bool pdl, cudaStream_t stream) {
   using C = WideCfg<TILE_N, STAGE_K, kPair, kDblTails>;
   Params p = p_in;
-  const int stages = wide_stages<C>(p.E, kFused);
+  const int stages = wide_stages<C>(p.E);
   if (stages < 2)
     return fail(PNV_ERR_INVALID_ARGUMENT, "group_mm: not enough shared memory for a %dx%d pipeline", TILE_N, STAGE_K);
   p.stages = stages;
-  p.prod_lanes = stages >= 8 ? 4 : stages >= 4 ? 2 : 1;
-  const size_t smem = 1024 + (size_t)stages * C::kStageBytes + (kFused ? C::kFusedOutBytes : C::kPlainOutBytes) +
-                      C::kBarrierBytes + 4 * (size_t)p.E;
+  const size_t smem = 1024 + (size_t)stages * C::kStageBytes + C::kOutBytes +
+                      C::kBarrierBytes + 8 * (size_t)p.E;
   static KernelSetup setup;
   int max_pairs = 0;
   if (int rc = prepare_kernel(group_mm_wide_kernel<TILE_N, STAGE_K, kFused, kPair, kDblTails>, setup, C::kThreads, smem, kPair,
@@ -906,12 +920,12 @@ int launch_wide_impl(const CUtensorMap& map_a, const CUtensorMap& map_b, const C
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = n_attr;
-  PNV_CUDA(cudaLaunchKernelEx(&cfg, group_mm_wide_kernel<TILE_N, STAGE_K, kFused, kPair, kDblTails>, map_a, map_b, map_b_tail, p));
+  PNV_CUDA(cudaLaunchKernelEx(&cfg, group_mm_wide_kernel<TILE_N, STAGE_K, kFused, kPair, kDblTails>, map_a, map_b, map_b_tail, map_out, p));
   return PNV_OK;
 }
 
 template <int TILE_N, int STAGE_K, bool kPair>
-int launch_wide(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_b_tail, Params& p, int sm_count,
+int launch_wide(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtensorMap& map_b_tail, const CUtensorMap& map_out, Params& p, int sm_count,
                 bool pdl, cudaStream_t stream) {
   // Pairs with 256-token tiles: when no expert can hold more than four token tiles, narrow tail tiles are a
   // large enough share of the work for the double-tail-item variant to pay for its overhead on the other items
@@ -919,13 +933,13 @@ int launch_wide(const CUtensorMap& map_a, const CUtensorMap& map_b, const CUtens
   if constexpr (kPair && TILE_N == 256) {
     if (p.b_tail != 0 && p.max_n <= 4 * TILE_N) {
       if (p.f_b_out != nullptr)
-        return launch_wide_impl<TILE_N, STAGE_K, true, kPair, true>(map_a, map_b, map_b_tail, p, sm_count, pdl, stream);
-      return launch_wide_impl<TILE_N, STAGE_K, false, kPair, true>(map_a, map_b, map_b_tail, p, sm_count, pdl, stream);
+        return launch_wide_impl<TILE_N, STAGE_K, true, kPair, true>(map_a, map_b, map_b_tail, map_out, p, sm_count, pdl, stream);
+      return launch_wide_impl<TILE_N, STAGE_K, false, kPair, true>(map_a, map_b, map_b_tail, map_out, p, sm_count, pdl, stream);
     }
   }
   if (p.f_b_out != nullptr)
-    return launch_wide_impl<TILE_N, STAGE_K, true, kPair>(map_a, map_b, map_b_tail, p, sm_count, pdl, stream);
-  return launch_wide_impl<TILE_N, STAGE_K, false, kPair>(map_a, map_b, map_b_tail, p, sm_count, pdl, stream);
+    return launch_wide_impl<TILE_N, STAGE_K, true, kPair>(map_a, map_b, map_b_tail, map_out, p, sm_count, pdl, stream);
+  return launch_wide_impl<TILE_N, STAGE_K, false, kPair>(map_a, map_b, map_b_tail, map_out, p, sm_count, pdl, stream);
 }
 
 // Tile variants.  The first eight names and ids are the reference's.  "1sm" variants run one CTA per
@@ -997,7 +1011,7 @@ struct FusedArgs {
   uint8_t* sfb_out = nullptr;
   const float* gscale = nullptr;
   int gpe = 0;
-  GatedAct act{PNV_ACT_SILU, 1.f, -1.f, nullptr};
+  GatedAct act{PNV_ACT_SILU, 1.f, -1.f, 0};
 };
 
 // The tile variants of the fused op, by the reference's names (csrc/sm100/tactics.cu:52-57).
@@ -1046,7 +1060,7 @@ int group_mm_common(void* out, const int32_t* row_map, const RowParts* out_parts
   p.row_map = row_map;
   p.out_parts = out_parts ? *out_parts : RowParts{};
   p.f_b_out = nullptr; p.f_sfb_out = nullptr; p.f_gscale = nullptr; p.f_gpe = 0; p.f_n = 0; p.f_n_kt = 0;
-  p.f_act = GatedAct{PNV_ACT_SILU, 1.f, -1.f, nullptr};
+  p.f_act = GatedAct{PNV_ACT_SILU, 1.f, -1.f, 0};
   if (fused != nullptr) {
     p.f_b_out = fused->b_out; p.f_sfb_out = fused->sfb_out; p.f_gscale = fused->gscale; p.f_gpe = fused->gpe;
     p.f_n = features / 2; p.f_n_kt = sf_k_atoms(features / 2); p.f_act = fused->act;
@@ -1058,8 +1072,8 @@ int group_mm_common(void* out, const int32_t* row_map, const RowParts* out_parts
   p.e_m_atoms = wd.m_e / 128;
   p.sfb_rt = sf_row_atoms(max_n);
   p.stages = 0;
-  p.prod_lanes = 1;
   p.b_tail = 0;
+  p.out_tma = 0;
   p.split_counters = nullptr;
   p.split_partials = nullptr;
 
@@ -1073,10 +1087,10 @@ int group_mm_common(void* out, const int32_t* row_map, const RowParts* out_parts
     stage_k = 512;
   }
   const bool pair = kind.two_sm && !narrow;
-  // The 256 x 256 pair kernel takes 512-K stages (three large ones instead of six) when K is long: every stage
-  // costs the lone issuing threads the same few hundred cycles whatever it holds, and a long K loop keeps a short
-  // ring busy (measured: K = 7168 -5 to -12 %, K = 3072 -10 %; K = 2048 +4 %, K = 768 +3 %).
-  if (pair && tile_n == 256 && stage_k == 256 && k >= 3072) stage_k = 512;
+  // The 256 x 256 pair kernel takes 512-K stages (three large ones instead of six) unless all of K fits a 256-K one:
+  // the weight copies are then 128 bytes wide, and the TMA's rate is per request (64-byte rows load no faster).
+  // Measured on the down GEMM of 32 experts x 2048 rows x 2048: 460 us against 556.
+  if (pair && tile_n == 256 && stage_k == 256 && k > 256) stage_k = 512;
   p.k_stages = ceil_div_i(k, stage_k);
   // the split schedule counts K stages in 32 bits
   const bool split_fits = (long long)experts * p.n_mt * p.k_stages < (1LL << 30);
@@ -1116,6 +1130,13 @@ int group_mm_common(void* out, const int32_t* row_map, const RowParts* out_parts
   }
 #endif
 
+  // plain outputs whose rows are 16-byte aligned: whole chunks of token rows leave through a tensor map
+  CUtensorMap map_out = map_b;
+  if (!narrow && fused == nullptr && row_map == nullptr && features % 8 == 0) {
+    if (int rc = make_map_out(&map_out, out, (uint64_t)features, (uint64_t)max_n, (uint64_t)experts, tile_n >= 128 ? 32 : 16)) return rc;
+    p.out_tma = 1;
+  }
+
   cudaStream_t s = (cudaStream_t)stream;
   const bool use_pdl = pdl != 0 && pdl_enabled();
   if (narrow) {
@@ -1123,16 +1144,16 @@ int group_mm_common(void* out, const int32_t* row_map, const RowParts* out_parts
     return launch_narrow<32, 512, 4>(map_a, map_b, p, sm_count, use_pdl, s);
   }
   switch (tile_n * 1000 + stage_k + (pair ? 1 : 0)) {
-    case 64256: return launch_wide<64, 256, false>(map_a, map_b, map_b_tail, p, sm_count, use_pdl, s);
-    case 64257: return launch_wide<64, 256, true>(map_a, map_b, map_b_tail, p, sm_count, use_pdl, s);
-    case 64512: return launch_wide<64, 512, false>(map_a, map_b, map_b_tail, p, sm_count, use_pdl, s);
-    case 64513: return launch_wide<64, 512, true>(map_a, map_b, map_b_tail, p, sm_count, use_pdl, s);
-    case 128256: return launch_wide<128, 256, false>(map_a, map_b, map_b_tail, p, sm_count, use_pdl, s);
-    case 128257: return launch_wide<128, 256, true>(map_a, map_b, map_b_tail, p, sm_count, use_pdl, s);
-    case 128512: return launch_wide<128, 512, false>(map_a, map_b, map_b_tail, p, sm_count, use_pdl, s);
-    case 256256: return launch_wide<256, 256, false>(map_a, map_b, map_b_tail, p, sm_count, use_pdl, s);
-    case 256257: return launch_wide<256, 256, true>(map_a, map_b, map_b_tail, p, sm_count, use_pdl, s);
-    case 256513: return launch_wide<256, 512, true>(map_a, map_b, map_b_tail, p, sm_count, use_pdl, s);
+    case 64256: return launch_wide<64, 256, false>(map_a, map_b, map_b_tail, map_out, p, sm_count, use_pdl, s);
+    case 64257: return launch_wide<64, 256, true>(map_a, map_b, map_b_tail, map_out, p, sm_count, use_pdl, s);
+    case 64512: return launch_wide<64, 512, false>(map_a, map_b, map_b_tail, map_out, p, sm_count, use_pdl, s);
+    case 64513: return launch_wide<64, 512, true>(map_a, map_b, map_b_tail, map_out, p, sm_count, use_pdl, s);
+    case 128256: return launch_wide<128, 256, false>(map_a, map_b, map_b_tail, map_out, p, sm_count, use_pdl, s);
+    case 128257: return launch_wide<128, 256, true>(map_a, map_b, map_b_tail, map_out, p, sm_count, use_pdl, s);
+    case 128512: return launch_wide<128, 512, false>(map_a, map_b, map_b_tail, map_out, p, sm_count, use_pdl, s);
+    case 256256: return launch_wide<256, 256, false>(map_a, map_b, map_b_tail, map_out, p, sm_count, use_pdl, s);
+    case 256257: return launch_wide<256, 256, true>(map_a, map_b, map_b_tail, map_out, p, sm_count, use_pdl, s);
+    case 256513: return launch_wide<256, 512, true>(map_a, map_b, map_b_tail, map_out, p, sm_count, use_pdl, s);
     default: break;
   }
   return fail(PNV_ERR_UNSUPPORTED, "group_mm: no kernel for tile %dx%d%s", tile_n, stage_k, pair ? " (pair)" : "");
@@ -1221,7 +1242,7 @@ extern "C" int pnv_group_mm_swiglu_quant(uint8_t* b_out, uint8_t* sfb_out, const
   PNV_REQUIRE((reinterpret_cast<uintptr_t>(b_out) | reinterpret_cast<uintptr_t>(sfb_out)) % 16 == 0,
               "group_mm operands must be 16-byte aligned");
   FusedArgs f;
-  if (int rc = make_gated_act(act_kind, beta, linear_beta, (cudaStream_t)stream, f.act)) return rc;
+  if (int rc = make_gated_act(act_kind, beta, linear_beta, f.act)) return rc;
   f.b_out = b_out; f.sfb_out = sfb_out; f.gscale = gscale; f.gpe = gscale_per_expert ? 1 : 0;
   PNV_REQUIRE(experts >= 1 && max_n >= 1, "experts and max_n must be positive");
   PNV_REQUIRE(sf_numel(max_n, features / 2, experts) < (1LL << 31), "sfb_out must be smaller than 2 GiB");

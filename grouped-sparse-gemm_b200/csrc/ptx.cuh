@@ -75,6 +75,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(bar, parity);
 }
+// The whole warp waits and gets one answer: the lanes of a converged warp can see the phase flip in different polls, and
+// a role whose lanes all follow the loop must not let some of them give up and others not.
+static __device__ __noinline__ bool mbar_wait_warp_slow(uint64_t* bar, uint32_t parity) {
+#pragma unroll 1
+  for (uint32_t i = 0; i < kMaxPolls; ++i) {
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    if (i > 64) __nanosleep(128);
+  }
+  return false;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return mbar_wait_warp_slow(bar, parity);
+}
 // The same loop with a caller-chosen poll budget (the self-test of the give-up path uses a short one).
 static __device__ __noinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity, uint32_t max_polls) {
 #pragma unroll 1
@@ -173,6 +187,15 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
       :
       : "r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
+}
+
+// 3-D tiled store shared -> global, tracked by the issuing thread's bulk-copy groups; elements outside the tensor are
+// not written.  Ordinary stores to the source need fence_proxy_async_smem() before the copy is issued.
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* src_smem, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(smem_u32(src_smem)), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
 }
 
 // Contiguous bulk copy shared -> global (both addresses 16-byte aligned, size a multiple of 16),
@@ -324,6 +347,31 @@ __host__ __device__ constexpr uint32_t mma_sp_nvf4_idesc(int n, int m = 128) {
   return (1u << 2) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
+// The matrix-fragment form: 16 lanes x 8 columns per step (16x256b), 4 or 2 steps.  Of step j a thread gets
+// r[4j], r[4j+1] = (lane l / 4, columns 8j + 2 (l % 4) and the next one) and r[4j+2], r[4j+3] = the same columns eight
+// lanes further on: two neighbouring columns of a row packed to 16 bits are an 8 x 8 fragment stmatrix can transpose.
+__device__ __forceinline__ void tc_ld_16x32(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tc_ld_16x16(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+// Four 8 x 8 fragments of 16-bit elements, each transposed on its way to shared memory: lane 8 i + j gives the
+// address of (transposed) row j of fragment i.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b),
+               "r"(c), "r"(d)
+               : "memory");
+}
 // tensor memory -> registers: this warp's 32 lanes x 32 consecutive 32-bit columns.
 __device__ __forceinline__ void tc_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(

@@ -12,8 +12,6 @@
 // scatter_quant_act is driven by a routing list instead (source token -> destination row), so its
 // scale buffer is pre-filled with a memset node and each warp quantizes 256 elements of one routed
 // row.
-#include <mutex>
-
 #include "common.cuh"
 
 namespace pnv {
@@ -97,15 +95,10 @@ quant_lines_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
         unpack8(g0, ga); unpack8(u0, ua);
         float gb[8], ub[8];
         unpack8(g1, gb); unpack8(u1, ub);
-        if (act.kind == PNV_ACT_SILU && act.silu_tab != nullptr) {   // straight-line: 16 independent lookups
 #pragma unroll
-          for (int i = 0; i < 8; ++i) { f0[i] = silu_mul(ga[i], ua[i], act.silu_tab); f1[i] = silu_mul(gb[i], ub[i], act.silu_tab); }
-        } else {
+        for (int i = 0; i < 8; ++i) f0[i] = gated_act(ga[i], ua[i], act);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) f0[i] = gated_act(ga[i], ua[i], act);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) f1[i] = gated_act(gb[i], ub[i], act);
-        }
+        for (int i = 0; i < 8; ++i) f1[i] = gated_act(gb[i], ub[i], act);
       }
     } else {
 #pragma unroll
@@ -409,64 +402,14 @@ int check_common(const void* x, const float* gscale, const int32_t* counts, int 
 
 }  // namespace
 
-// ---- SiLU table ---------------------------------------------------------------------------------
-// 128 KiB inside the library, one copy per device, filled on first use by a kernel on the caller's
-// stream; later callers on other streams wait for that kernel through an event (no host wait).  A
-// first use inside a stream capture puts the fill kernel into the capture instead (it is
-// idempotent), so a graph never depends on work outside it.
-static __device__ uint16_t g_silu_tab[65536];
-bool g_silu_table_on = true;
+static bool g_silu_short = true;
 
-__global__ void silu_table_kernel(uint16_t* tab) {
-  const unsigned bits = blockIdx.x * blockDim.x + threadIdx.x;
-  if (bits < 65536u) tab[bits] = (uint16_t)(__float_as_uint(silu_direct(__uint_as_float(bits << 16))) >> 16);
-}
-
-int silu_table(cudaStream_t stream, const uint16_t** out) {
-  constexpr int kMaxDevices = 64;
-  static std::mutex mu;
-  static int state[kMaxDevices] = {};          // 0 nothing yet, 1 fill launched, 2 fill known complete
-  static uint16_t* ptr[kMaxDevices] = {};
-  static cudaEvent_t filled[kMaxDevices] = {};
-  int dev = 0;
-  PNV_CUDA(cudaGetDevice(&dev));
-  PNV_REQUIRE(dev >= 0 && dev < kMaxDevices, "device index %d out of range", dev);
-  std::lock_guard<std::mutex> lock(mu);
-  if (ptr[dev] == nullptr) {
-    void* sym = nullptr;
-    PNV_CUDA(cudaGetSymbolAddress(&sym, g_silu_tab));
-    ptr[dev] = static_cast<uint16_t*>(sym);
-  }
-  *out = ptr[dev];
-  if (state[dev] == 2) return PNV_OK;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  PNV_CUDA(cudaStreamIsCapturing(stream, &cap));
-  const bool capturing = cap != cudaStreamCaptureStatusNone;
-  if (state[dev] == 1 && !capturing) {
-    cudaError_t q = cudaEventQuery(filled[dev]);
-    if (q == cudaSuccess) { state[dev] = 2; return PNV_OK; }
-    if (q != cudaErrorNotReady) return fail(PNV_ERR_CUDA, "cudaEventQuery failed: %s", cudaGetErrorString(q));
-    PNV_CUDA(cudaStreamWaitEvent(stream, filled[dev], 0));
-    return PNV_OK;
-  }
-  silu_table_kernel<<<256, 256, 0, stream>>>(ptr[dev]);
-  PNV_CUDA(cudaGetLastError());
-  if (!capturing && state[dev] == 0) {
-    PNV_CUDA(cudaEventCreateWithFlags(&filled[dev], cudaEventDisableTiming));
-    PNV_CUDA(cudaEventRecord(filled[dev], stream));
-    state[dev] = 1;
-  }
-  return PNV_OK;
-}
-
-int make_gated_act(int act_kind, float beta, float linear_beta, cudaStream_t stream, GatedAct& out) {
+int make_gated_act(int act_kind, float beta, float linear_beta, GatedAct& out) {
   if (act_kind == PNV_ACT_SILU) {
-    out = GatedAct{PNV_ACT_SILU, 1.0f, -1.0f, nullptr};
-    if (g_silu_table_on)
-      if (int rc = silu_table(stream, &out.silu_tab)) return rc;
+    out = GatedAct{PNV_ACT_SILU, 1.0f, -1.0f, g_silu_short ? 0 : 1};
   } else if (act_kind == PNV_ACT_SITU) {
     PNV_REQUIRE(beta > 0, "situ: beta must be positive, got %g", (double)beta);
-    out = GatedAct{PNV_ACT_SITU, beta, linear_beta, nullptr};
+    out = GatedAct{PNV_ACT_SITU, beta, linear_beta, 0};
   } else {
     return fail(PNV_ERR_INVALID_ARGUMENT, "activation must be 'silu' or 'situ', got kind %d", act_kind);
   }
@@ -482,7 +425,7 @@ extern "C" int pnv_quant_act(const void* x, const float* gscale, int gscale_per_
                              uint8_t* sfb, int sm_count, pnv_stream_t stream) {
   if (int rc = check_common(x, gscale, counts, experts, max_n, k, b_act, sfb, "K")) return rc;
   long long lines = sf_numel(max_n, k, experts) / 16;
-  GatedAct act{PNV_ACT_SILU, 1.f, -1.f, nullptr};
+  GatedAct act{PNV_ACT_SILU, 1.f, -1.f, 0};
   PNV_CUDA(launch_pdl(quant_lines_kernel<kPlain>, dim3(grid_for(lines, sm_count)), dim3(kThreads), 0,
                       (cudaStream_t)stream, pdl_enabled(), (const __nv_bfloat16*)x, gscale,
                       gscale_per_expert, counts, experts, max_n, k, 0, act, b_act, sfb));
@@ -495,7 +438,7 @@ extern "C" int pnv_silu_mul_quant_act(const void* x2, const float* gscale, int g
                                       uint8_t* b_act, uint8_t* sfb, int sm_count,
                                       pnv_stream_t stream) {
   GatedAct act;
-  if (int rc = make_gated_act(act_kind, beta, linear_beta, (cudaStream_t)stream, act)) return rc;
+  if (int rc = make_gated_act(act_kind, beta, linear_beta, act)) return rc;
   if (int rc = check_common(x2, gscale, counts, experts, max_n, n, b_act, sfb, "intermediate width N"))
     return rc;
   long long lines = sf_numel(max_n, n, experts) / 16;
@@ -532,7 +475,7 @@ extern "C" int pnv_scatter_quant_act(const void* a1, const int64_t* flat_tok,
 extern "C" int pnv_gated_act(const void* x2, int64_t rows, int n, int interleaved, int act_kind,
                              float beta, float linear_beta, void* y, pnv_stream_t stream) {
   GatedAct act;
-  if (int rc = make_gated_act(act_kind, beta, linear_beta, (cudaStream_t)stream, act)) return rc;
+  if (int rc = make_gated_act(act_kind, beta, linear_beta, act)) return rc;
   PNV_REQUIRE(x2 && y, "null pointer argument");
   PNV_REQUIRE(n > 0 && n % kSfBlock == 0, "intermediate width N must be a multiple of %d, got %d", kSfBlock, n);
   if (rows <= 0) return PNV_OK;
@@ -603,7 +546,7 @@ extern "C" int pnv_scatter_fp4_planned(const uint8_t* q, const uint8_t* q_sf, co
 }
 
 extern "C" int pnv_set_silu_table(int enabled) {
-  g_silu_table_on = enabled != 0;
+  g_silu_short = enabled != 0;
   return PNV_OK;
 }
 

@@ -392,7 +392,7 @@ def moe_finalize(out, fused, route_dest, topk_weights):
 
 
 def set_silu_table(enabled):
-    """Testing aid: evaluate SiLU through the library's lookup table (default) or directly."""
+    """Testing aid: evaluate SiLU in the library's short form (default) or by the expression itself."""
     _cabi.check(_lib.pnv_set_silu_table(1 if enabled else 0))
 
 

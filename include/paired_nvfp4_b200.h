@@ -231,9 +231,10 @@ int pnv_zero_rows_parts(void* const* parts, int n_parts, int64_t rows_per_part, 
 int pnv_gated_act(const void* x2, int64_t rows, int n, int interleaved, int act_kind, float beta,
                   float linear_beta, void* y, pnv_stream_t stream);
 
-/* Testing aid (no reference counterpart): SiLU is evaluated through a 65536-entry table of bf16(g / (1 + expf(-g)))
- * built into the library and filled on the device with that same expression; 0 switches the table off so that a
- * test can compare both paths bit for bit.  Process-wide; default on. */
+/* Testing aid (no reference counterpart): SiLU is evaluated in a short form that gives the bits of
+ * bf16(g / (1 + expf(-g))) for every bf16 gate; 0 evaluates that expression itself instead, so that a test can
+ * compare the two bit for bit.  (The name dates from a table that once stood in for the short form.)  Process-wide;
+ * default on. */
 int pnv_set_silu_table(int enabled);
 
 /* ---- grouped GEMM ------------------------------------------------------------------------- */
