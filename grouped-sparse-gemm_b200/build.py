@@ -1,9 +1,10 @@
-"""Build libpaired_nvfp4_b200.so in-tree with nvcc for sm_100a (no torch dependency).
+"""Build libpaired_nvfp4_b200.so in-tree with nvcc for sm_100a (no torch dependency), then the operator layer
+libpaired_nvfp4_torch.so (C++ against torch's headers) that registers torch.ops.paired_nvfp4.* on top of it.
 
     python grouped-sparse-gemm_b200/build.py [--force] [--ptxas-v]
 
-The library lands in grouped-sparse-gemm_b200/paired_nvfp4_kernels/, next to the Python package
-that loads it.  PAIRED_NVFP4_PTXAS_V=1 (or --ptxas-v) prints registers / spills / shared memory.
+Both land in grouped-sparse-gemm_b200/paired_nvfp4_kernels/, next to the Python package
+that loads them.  PAIRED_NVFP4_PTXAS_V=1 (or --ptxas-v) prints registers / spills / shared memory.
 """
 import os
 import subprocess
@@ -12,36 +13,62 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "paired_nvfp4_kernels", "libpaired_nvfp4_b200.so")
+TORCH_SRC = os.path.join(CSRC, "torch_ops.cpp")
+TORCH_OUT = os.path.join(HERE, "paired_nvfp4_kernels", "libpaired_nvfp4_torch.so")
+HEADER = os.path.join(os.path.dirname(HERE), "include", "paired_nvfp4_b200.h")
 SOURCES = ["abi.cu", "quant.cu", "compress.cu", "routing.cu", "group_mm.cu"]
 
 
 def _inputs():
-    files = [os.path.join(CSRC, f) for f in os.listdir(CSRC)]
-    files.append(os.path.join(os.path.dirname(HERE), "include", "paired_nvfp4_b200.h"))
-    return files
+    return [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cu", ".cuh"))] + [HEADER]
 
 
-def up_to_date():
-    if not os.path.exists(OUT):
+def up_to_date(out, inputs):
+    if not os.path.exists(out):
         return False
-    t = os.path.getmtime(OUT)
-    return all(os.path.getmtime(f) <= t for f in _inputs())
+    t = os.path.getmtime(out)
+    return all(os.path.getmtime(f) <= t for f in inputs)
 
 
-def build(force=False, ptxas_v=False, verbose=True):
-    if not force and up_to_date():
-        return OUT
-    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    cmd = [nvcc, "-shared", "-Xcompiler", "-fPIC", "-std=c++17", "-O3", "-lineinfo",
-           "-gencode", "arch=compute_100a,code=sm_100a", "-o", OUT]
-    if ptxas_v or os.environ.get("PAIRED_NVFP4_PTXAS_V") == "1":
-        cmd += ["-Xptxas", "-v"]
-    cmd += os.environ.get("PAIRED_NVFP4_NVCC_FLAGS", "").split()      # developer builds, e.g. -DPNV_WIDE_PROFILE
-    cmd += [os.path.join(CSRC, s) for s in SOURCES]
+def _run(cmd, verbose):
     if verbose:
         print(" ".join(cmd), flush=True)
     subprocess.run(cmd, check=True)
+
+
+def _cuda_home():
+    return os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+def build(force=False, ptxas_v=False, verbose=True):
+    if force or not up_to_date(OUT, _inputs()):
+        nvcc = os.environ.get("NVCC", os.path.join(_cuda_home(), "bin", "nvcc"))
+        cmd = [nvcc, "-shared", "-Xcompiler", "-fPIC", "-std=c++17", "-O3", "-lineinfo",
+               "-gencode", "arch=compute_100a,code=sm_100a", "-o", OUT]
+        if ptxas_v or os.environ.get("PAIRED_NVFP4_PTXAS_V") == "1":
+            cmd += ["-Xptxas", "-v"]
+        cmd += os.environ.get("PAIRED_NVFP4_NVCC_FLAGS", "").split()      # developer builds, e.g. -DPNV_WIDE_PROFILE
+        _run(cmd + [os.path.join(CSRC, s) for s in SOURCES], verbose)
+    build_torch_ops(force, verbose)
     return OUT
+
+
+def build_torch_ops(force=False, verbose=True):
+    if not force and up_to_date(TORCH_OUT, [TORCH_SRC, HEADER]):
+        return TORCH_OUT
+    import torch
+    root = os.path.dirname(torch.__file__)
+    lib = os.path.join(root, "lib")
+    # the g++ on PATH, not $CXX: libstdc++ has to be the shared one that torch uses (a second, static copy inside this
+    # library crashed while formatting an error message)
+    _run(["g++", "-shared", "-fPIC", "-std=c++17", "-O2", "-fvisibility=hidden",
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+          "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+          "-isystem", os.path.join(_cuda_home(), "include"), TORCH_SRC, "-o", TORCH_OUT,
+          "-L" + lib, "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10",
+          "-L" + os.path.dirname(OUT), "-lpaired_nvfp4_b200", "-L" + os.path.join(_cuda_home(), "lib64"), "-lcudart",
+          "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + lib], verbose)
+    return TORCH_OUT
 
 
 if __name__ == "__main__":

@@ -1,12 +1,12 @@
 """paired_nvfp4_kernels for B200 (sm_100a): paired-4:8 sparse NVFP4 grouped MoE GEMM ops.
 
 Importing this package loads ``libpaired_nvfp4_b200.so`` (hand-written sm_100a CUDA behind a C ABI)
-and registers ``torch.ops.paired_nvfp4.*`` with the reference project's operator schemas
-(csrc/ops.cu:739-773), so code written against the reference's package runs unchanged.  The helper
+and ``libpaired_nvfp4_torch.so``, which registers ``torch.ops.paired_nvfp4.*`` with the reference project's
+operator schemas (csrc/ops.cu:739-773), so code written against the reference's package runs unchanged.  The helper
 surface of the reference's ``paired_nvfp4_kernels/__init__.py`` (tactic enumeration, the gate/up
 interleave permutation, availability probes) is provided under the same names.
 
-There is no CPU or eager-PyTorch fallback: without the compiled library the import fails.
+There is no CPU or eager-PyTorch fallback: without the compiled libraries the import fails.
 """
 import torch
 
@@ -29,83 +29,9 @@ __all__ = [
 
 _LOADED_SM = 100
 
-# (config_id, cluster_m, cluster_n): also the schema defaults of torch.ops.paired_nvfp4.group_mm
+# (config_id, cluster_m, cluster_n): also the schema defaults of torch.ops.paired_nvfp4.group_mm (csrc/torch_ops.cpp)
 DEFAULT_TACTIC = (0, 2, 1)
 _CLUSTER_DIMS = (1, 2, 4)
-
-
-def _register():
-    lib = torch.library.Library("paired_nvfp4", "DEF")
-    lib.define("compress(Tensor w_packed, Tensor w_blockscale, int k) -> (Tensor, Tensor, Tensor)")
-    lib.define("quant_act(Tensor x, Tensor gscale, Tensor expert_num_tokens, int features) -> (Tensor, Tensor)")
-    lib.define("silu_mul_quant_act(Tensor x2, Tensor gscale, Tensor expert_num_tokens, int features, "
-               "bool interleaved=False, str activation=\"silu\", float beta=1.0, float linear_beta=-1.0) "
-               "-> (Tensor, Tensor)")
-    lib.define("scatter_quant_act(Tensor a1, Tensor flat_tok, Tensor dest_global, Tensor? topk_weights, "
-               "Tensor gscale, Tensor expert_num_tokens, int cap) -> (Tensor, Tensor)")
-    lib.define("dispatch_plan(Tensor topk_ids, int first_expert, int num_local_experts, int cap) "
-               "-> (Tensor, Tensor, Tensor, Tensor)")
-    lib.define("scatter_quant_act_planned(Tensor a1, Tensor src_tok, Tensor src_route, Tensor? topk_weights, "
-               "Tensor gscale, Tensor expert_num_tokens, int cap) -> (Tensor, Tensor)")
-    lib.define("quant_rows(Tensor x, Tensor gscale) -> (Tensor, Tensor)")
-    lib.define("scatter_fp4_planned(Tensor q, Tensor q_sf, Tensor src_tok, Tensor expert_num_tokens, int cap) "
-               "-> (Tensor, Tensor)")
-    lib.define("moe_finalize(Tensor(a!) out, Tensor fused, Tensor route_dest, Tensor? topk_weights) -> ()")
-    lib.define("gather_rows(Tensor src, Tensor idx) -> Tensor")
-    lib.define("pack_wire_rows(Tensor q, Tensor q_sf, Tensor topk_ids, Tensor slot_tok, Tensor slot_route, "
-               "Tensor slab_counts, int slab, int experts_per_rank) -> Tensor")
-    lib.define("scatter_fp4_wire(Tensor wire, int k, Tensor src_tok, Tensor expert_num_tokens, int cap) "
-               "-> (Tensor, Tensor)")
-    lib.define("group_mm(Tensor(a!) out, Tensor a_comp, Tensor e_meta, Tensor sfa, Tensor b_act, Tensor sfb, "
-               "Tensor alphas, Tensor expert_num_tokens, int features, int k, "
-               f"int config_id={DEFAULT_TACTIC[0]}, int cluster_m={DEFAULT_TACTIC[1]}, "
-               f"int cluster_n={DEFAULT_TACTIC[2]}) -> ()")
-    lib.define("group_mm_rows(Tensor(a!) out, Tensor row_map, Tensor a_comp, Tensor e_meta, Tensor sfa, Tensor b_act, "
-               "Tensor sfb, Tensor alphas, Tensor expert_num_tokens, int features, int k, "
-               f"int config_id={DEFAULT_TACTIC[0]}, int cluster_m={DEFAULT_TACTIC[1]}, "
-               f"int cluster_n={DEFAULT_TACTIC[2]}) -> ()")
-    lib.define("zero_rows(Tensor(a!) dst, Tensor flags) -> ()")
-    lib.define("group_mm_rows_parts(Tensor(a!)[] out_parts, Tensor row_map, Tensor a_comp, Tensor e_meta, Tensor sfa, "
-               "Tensor b_act, Tensor sfb, Tensor alphas, Tensor expert_num_tokens, int features, int k, "
-               f"int config_id={DEFAULT_TACTIC[0]}, int cluster_m={DEFAULT_TACTIC[1]}, "
-               f"int cluster_n={DEFAULT_TACTIC[2]}) -> ()")
-    lib.define("zero_rows_parts(Tensor(a!)[] parts, Tensor flags) -> ()")
-    lib.define("pack_wire_rows_parts(Tensor q, Tensor q_sf, Tensor topk_ids, Tensor slot_tok, Tensor slot_route, "
-               "Tensor slab_counts, int slab, int experts_per_rank, Tensor(a!)[] wire_parts) -> ()")
-    lib.define("group_mm_configs() -> str[]")
-    lib.define("group_mm_swiglu_quant(Tensor a_comp, Tensor e_meta, Tensor sfa, Tensor b_act, Tensor sfb, "
-               "Tensor alphas, Tensor expert_num_tokens, Tensor gscale, int features, int k, int config_id=0, "
-               f"int cluster_m={DEFAULT_TACTIC[1]}, int cluster_n={DEFAULT_TACTIC[2]}, "
-               "str activation=\"silu\", float beta=1.0, float linear_beta=-1.0) -> (Tensor, Tensor)")
-    lib.define("group_mm_swiglu_configs() -> str[]")
-    lib.define("gated_act(Tensor x2, bool interleaved=False, str activation=\"silu\", float beta=1.0, "
-               "float linear_beta=-1.0) -> Tensor")
-    lib.impl("compress", ops.compress, "CUDA")
-    lib.impl("quant_act", ops.quant_act, "CUDA")
-    lib.impl("silu_mul_quant_act", ops.silu_mul_quant_act, "CUDA")
-    lib.impl("scatter_quant_act", ops.scatter_quant_act, "CUDA")
-    lib.impl("dispatch_plan", ops.dispatch_plan, "CUDA")
-    lib.impl("scatter_quant_act_planned", ops.scatter_quant_act_planned, "CUDA")
-    lib.impl("quant_rows", ops.quant_rows, "CUDA")
-    lib.impl("scatter_fp4_planned", ops.scatter_fp4_planned, "CUDA")
-    lib.impl("moe_finalize", ops.moe_finalize, "CUDA")
-    lib.impl("gather_rows", ops.gather_rows, "CUDA")
-    lib.impl("pack_wire_rows", ops.pack_wire_rows, "CUDA")
-    lib.impl("scatter_fp4_wire", ops.scatter_fp4_wire, "CUDA")
-    lib.impl("group_mm", ops.group_mm, "CUDA")
-    lib.impl("group_mm_rows", ops.group_mm_rows, "CUDA")
-    lib.impl("zero_rows", ops.zero_rows, "CUDA")
-    lib.impl("group_mm_rows_parts", ops.group_mm_rows_parts, "CUDA")
-    lib.impl("zero_rows_parts", ops.zero_rows_parts, "CUDA")
-    lib.impl("pack_wire_rows_parts", ops.pack_wire_rows_parts, "CUDA")
-    lib.impl("gated_act", ops.gated_act, "CUDA")
-    lib.impl("group_mm_swiglu_quant", ops.group_mm_swiglu_quant, "CUDA")
-    lib.impl("group_mm_configs", ops.group_mm_configs, "CompositeExplicitAutograd")
-    lib.impl("group_mm_swiglu_configs", ops.group_mm_swiglu_configs, "CompositeExplicitAutograd")
-    return lib
-
-
-_LIB = _register()   # kept alive for the life of the process
 
 
 def _current_sm():
