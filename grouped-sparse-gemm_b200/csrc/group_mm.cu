@@ -4,22 +4,20 @@
 // Persistent kernels, one CTA per SM.  group_mm_kernel (this file) runs the 16- and 32-token tiles of
 // decode-sized problems (max_n <= 32); group_mm_wide_kernel (group_mm_wide.cuh) the 64- to 256-token
 // tiles, on one CTA per tile ("1sm" variants) or on a CTA pair per tile ("2sm" variants).
-// Narrow kernel, four warp roles (6 + ISSUERS warps):
-//   warp 0 (one lane)  tile producer: per K stage, the TMA tile loads of the compressed weights and
+// Narrow kernel, four warp roles (6 + ISSUERS warps).  The single-warp roles run warp-uniform: all 32 lanes follow the
+// loop and an elected one issues (operands in uniform registers; a lane that a thread-index test picked pays 85 cycles
+// and more of set-up per TMA, bulk-copy or tcgen05 instruction).
+//   warp 0             tile producer: per K stage, the TMA tile loads of the compressed weights and
 //                      of the activations (one tensor map each covers every expert; 128-byte swizzle)
-//   warp 1 (two lanes) side producer: plain bulk copies of the metadata atoms and of the SFA / SFB
+//   warp 1             side producer: plain bulk copies of the metadata atoms and of the SFA / SFB
 //                      scale atoms, which sit in global memory in exactly the shape tcgen05.cp
 //                      consumes and so need no tensor map;
-//   ISSUERS warps      MMA issuers (one lane each): issuer j owns a fixed slice of every stage's
-//   (one lane each)    128-K blocks.  It copies their metadata and scales into tensor memory
+//   ISSUERS warps      MMA issuers: issuer j owns a fixed slice of every stage's
+//                      128-K blocks.  It copies their metadata and scales into tensor memory
 //                      (tcgen05.cp), issues one tcgen05.mma.sp block-scaled instruction
 //                      (128 x TILE_N x 128) per block into its own partial accumulator, and commits:
 //                      to the stage's "empty" barrier, and after the tile's last stage to the
-//                      accumulator's "full" barrier.  A tcgen05 operation holds its issuing thread
-//                      for about as long as it executes (MMA 66-160 cycles, copy 35-50) and the
-//                      thread's own instructions in between add to that, so with narrow tiles a
-//                      single issuer, not memory, would bound the kernel; issuers in different
-//                      warps overlap.
+//                      accumulator's "full" barrier.  Issuers in different warps overlap.
 //   last 4 warps       epilogue: tcgen05.ld the partial accumulators 32 token columns at a time, add
 //                      them, scale by alpha[e], round to bf16, transpose through shared memory and
 //                      store 16 bytes per thread, 256 contiguous bytes per output row; or, in the
@@ -27,8 +25,8 @@
 // Accumulators are double buffered, so the epilogue of one tile overlaps the main loop of the next.
 //
 // Tile schedule: every role walks the same list on its own, derived on the device from
-// counts[]: experts in order, each contributing ceil(M/128) * ceil(counts[e]/TILE_N) tiles
-// (M tile fastest); CTA b takes tiles b, b + grid, ...  No host read of counts, no scheduler
+// counts[]: active experts in order, each contributing ceil(M/128) tiles; CTA b takes tiles
+// b, b + grid, ... (or a range of K stages, see UnitWalk).  No host read of counts, no scheduler
 // state in global memory: the launch is fixed-shape and safe to capture in a CUDA graph.
 //
 // Every mbarrier wait is bounded; a wait that gives up records a code in g_status, and every role
@@ -55,7 +53,7 @@ constexpr int kColSfa = 464;                 //   weight scales (4 per K-block)
 constexpr int kColSfb = 480;                 //   activation scales (4 or 8 per K-block)
 constexpr int kOutRow = kTileM + 8;          // padded row of the epilogue transpose buffer (bank spread)
 constexpr int kOutStageBytes = 2 * 32 * kOutRow * 2;   // 2 x [32 token columns][136] bf16
-constexpr int kMaxExperts = 2048;            // bounds the shared-memory copy of counts
+constexpr int kMaxExperts = 2048;            // bounds the shared-memory copies of counts
 constexpr int kSmemLimit = 227 * 1024;
 
 enum Status : int {
@@ -84,7 +82,7 @@ struct Cfg {
   static constexpr int kSfbRowAtoms = TILE_N > 128 ? 2 : 1;
   static constexpr int kSfbBytes = kSfaBytes * kSfbRowAtoms;
   static constexpr int kStageBytes = kABytes + kBBytes + kEBytes + kSfaBytes + kSfbBytes;
-  static constexpr int kFixedBytes = 1024 + kOutStageBytes + 256 + 4 * kMaxExperts;
+  static constexpr int kFixedBytes = 1024 + kOutStageBytes + 256 + 6 * kMaxExperts;
   static constexpr int kStages = (kSmemLimit - kFixedBytes) / kStageBytes;
   static constexpr int kAccStages = TILE_N == 256 ? 1 : 2;
   static constexpr int kSfbColsPerAtom = 4 * kSfbRowAtoms;
@@ -146,32 +144,6 @@ __device__ __forceinline__ __nv_bfloat16* mapped_row(const Params& p, long long 
   return reinterpret_cast<__nv_bfloat16*>(part_row(p.out_parts, to, 2LL * p.M));
 }
 
-// The walk over (expert, n tile, m tile) shared by all roles.
-struct TileWalk {
-  const int* cnt;    // shared-memory copy of counts, clamped to [0, max_n]
-  int E, n_mt, e;
-  long long base;    // first tile index of expert e
-  long long tiles_e;
-  template <int TILE_N>
-  __device__ void init(const int* s_counts, int E_, int n_mt_) {
-    cnt = s_counts; E = E_; n_mt = n_mt_; e = 0; base = 0;
-    tiles_e = (long long)n_mt * ceil_div_i(cnt[0], TILE_N);
-  }
-  template <int TILE_N>
-  __device__ bool seek(long long t, int& mt, int& nt) {
-    while (t >= base + tiles_e) {
-      base += tiles_e;
-      if (++e >= E) return false;
-      tiles_e = (long long)n_mt * ceil_div_i(cnt[e], TILE_N);
-    }
-    // an expert's own tile count fits 32 bits (its output alone would otherwise exceed the device)
-    const unsigned local = (unsigned)(t - base);
-    nt = (int)(local / (unsigned)n_mt);
-    mt = (int)(local - (unsigned)nt * (unsigned)n_mt);
-    return true;
-  }
-};
-
 // Narrow kernel: the work of one CTA as a list of units (tile, K stages [ks0, ks1)).
 //   unsplit   CTA b takes whole tiles b, b + grid, ...
 //   split K   the K stages of all tiles, laid end to end, are cut into `grid` equal ranges; CTA b takes range b, so
@@ -181,26 +153,39 @@ struct TileWalk {
 //             range finishing an earlier tile, slot 2b, and the tail starting a later one, slot 2b + 1) and bumps
 //             the tile's arrival counter; whichever CTA arrives last adds the tile's slots in K order, so the sum
 //             does not depend on timing, and runs the ordinary epilogue.  Nobody waits for anybody.
+//             Only where that saves kSplitSaves stages per CTA or more: the partial sums' way through memory and the
+//             arrival counters cost about as long as that many stages.
+// A narrow tile holds all tokens of its expert, so tile t is M tile t % n_mt of active expert t / n_mt: with the list of
+// active experts (counts > 0) in shared memory no role walks over the idle ones.  One token on 8 of 128 experts, 2048 x
+// 1536 and 768 x 2048 weights: 16 and 17 us per GEMM with that walk and with K always split, 6.5 and 5.4 us now.
+constexpr int kSplitSaves = 6;
 struct UnitWalk {
-  TileWalk tw;
+  const unsigned short* active;      // the active experts in order
+  unsigned n_tiles, n_mt;
+  int e;             // expert of the current unit
   bool split;
   unsigned ksn, grid;
   // split: K stages of all tiles (the host bounds it below 2^31), and the cut: the first `rem` CTAs take
-  // `quot` + 1 stages, the others `quot` -- no division per lookup (a lone thread pays hundreds of cycles for one)
+  // `quot` + 1 stages, the others `quot` -- no division per lookup
   unsigned total, quot, rem;
   unsigned pos, hi;  // split: this CTA's range; unsplit: pos is the next tile
-  template <int TILE_N>
-  __device__ void init(const int* s_counts, int E, int n_mt, int k_stages, long long n_tiles, bool split_) {
-    tw.init<TILE_N>(s_counts, E, n_mt);
-    split = split_; ksn = (unsigned)k_stages; grid = gridDim.x;
-    if (split) {
-      total = (unsigned)n_tiles * ksn;
-      quot = total / grid;
-      rem = total - quot * grid;
-      pos = range_lo(blockIdx.x);
-      hi = range_lo(blockIdx.x + 1);
-    } else {
-      total = quot = rem = 0; pos = blockIdx.x; hi = 0;
+  __device__ void init(const unsigned short* active_, unsigned n_active, int n_mt_, int k_stages, bool may_split) {
+    active = active_; n_mt = (unsigned)n_mt_; n_tiles = n_active * n_mt; e = 0;
+    ksn = (unsigned)k_stages; grid = gridDim.x;
+    split = false;
+    total = quot = rem = 0; pos = blockIdx.x; hi = 0;
+    // Whole tiles are kept where there are 1.5 or more per CTA: the partial sums and their reduction then cost more than
+    // the imbalance they remove (measured on an 8-expert decode step: 63.5 / 37.1 us split against 58.9 / 35.2 us whole)
+    if (may_split && 2 * n_tiles < 3 * grid) {
+      const unsigned sum = n_tiles * ksn, q = sum / grid;
+      if (ksn >= q + 1 + kSplitSaves) {
+        split = true;
+        total = sum;
+        quot = q;
+        rem = total - quot * grid;
+        pos = range_lo(blockIdx.x);
+        hi = range_lo(blockIdx.x + 1);
+      }
     }
   }
   __device__ unsigned range_lo(unsigned b) const { return quot * b + min(b, rem); }
@@ -210,22 +195,22 @@ struct UnitWalk {
     return x < big ? x / (quot + 1) : rem + (x - big) / quot;
   }
   // next unit of this CTA; slot = workspace slot of a partial unit
-  template <int TILE_N>
-  __device__ bool next(long long& tile, int& mt, int& nt, int& ks0, int& ks1, int& slot) {
+  __device__ bool next(unsigned& tile, int& mt, int& ks0, int& ks1, int& slot) {
     if (!split) {
-      if (!tw.seek<TILE_N>(pos, mt, nt)) return false;
+      if (pos >= n_tiles) return false;
       tile = pos; ks0 = 0; ks1 = (int)ksn; slot = 0;
       pos += grid;
-      return true;
+    } else {
+      if (pos >= hi) return false;
+      tile = pos / ksn;
+      ks0 = (int)(pos - tile * ksn);
+      ks1 = (int)min(ksn, (unsigned)ks0 + (hi - pos));
+      slot = 2 * (int)blockIdx.x + (pos == range_lo(blockIdx.x) ? 0 : 1);
+      pos += (unsigned)(ks1 - ks0);
     }
-    if (pos >= hi) return false;
-    const unsigned t = pos / ksn;
-    tile = t;
-    ks0 = (int)(pos - t * ksn);
-    ks1 = (int)min(ksn, (unsigned)ks0 + (hi - pos));
-    slot = 2 * (int)blockIdx.x + (pos == range_lo(blockIdx.x) ? 0 : 1);
-    tw.seek<TILE_N>(tile, mt, nt);     // inside the list by construction
-    pos += (unsigned)(ks1 - ks0);
+    const unsigned i = tile / n_mt;
+    mt = (int)(tile - i * n_mt);
+    e = active[i];
     return true;
   }
 };
@@ -251,6 +236,7 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   uint64_t* acc_empty = acc_full + C::kAccStages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + C::kAccStages);
   int* s_counts = reinterpret_cast<int*>(smem + C::kStages * C::kStageBytes + kOutStageBytes + 256);
+  unsigned short* s_active = reinterpret_cast<unsigned short*>(s_counts + p.E);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -259,8 +245,8 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   if (threadIdx.x == 0) {
     ptx::prefetch_tensormap(&map_a);
     ptx::prefetch_tensormap(&map_b);
-    // arrivals on a stage's full barrier: the tile producer and the two bulk-copy lanes
-    for (int s = 0; s < C::kStages; ++s) { ptx::mbar_init(full_bar + s, 3); ptx::mbar_init(empty_bar + s, ISSUERS); }
+    // arrivals on a stage's full barrier: the tile producer and the side producer
+    for (int s = 0; s < C::kStages; ++s) { ptx::mbar_init(full_bar + s, 2); ptx::mbar_init(empty_bar + s, ISSUERS); }
     for (int a = 0; a < C::kAccStages; ++a) {
       ptx::mbar_init(acc_full + a, ISSUERS);
       ptx::mbar_init(acc_empty + a, kEpilogueThreads);
@@ -279,42 +265,41 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // every thread counts the tiles of the launch (the split schedule is cut from their total)
-  long long n_tiles = 0;
-  if (p.split_counters != nullptr) {
-    for (int e = lane; e < p.E; e += 32) n_tiles += (long long)p.n_mt * ceil_div_i(s_counts[e], TILE_N);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n_tiles += __shfl_xor_sync(0xffffffffu, n_tiles, o);
+  // The list of active experts.  Every warp builds all of it: they write the same values to the same places, so a warp
+  // needs no barrier to read what it has written itself.
+  unsigned n_active = 0;
+  for (int e0 = 0; e0 < p.E; e0 += 32) {
+    const bool on = e0 + lane < p.E && s_counts[e0 + lane] > 0;
+    const unsigned m = __ballot_sync(0xffffffffu, on);
+    if (on) s_active[n_active + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(e0 + lane);
+    n_active += __popc(m);
   }
+  __syncwarp();
 
-  // K is split only when whole tiles would leave SMs idle or the last wave thin (fewer than 1.5 tiles per CTA):
-  // with more tiles than that the partial sums and their reduction cost more than the imbalance they remove
-  // (measured on an 8-expert decode step: 63.5 / 37.1 us split against 58.9 / 35.2 us whole)
   UnitWalk walk;
-  walk.init<TILE_N>(s_counts, p.E, p.n_mt, p.k_stages, n_tiles,
-                    p.split_counters != nullptr && 2 * n_tiles < 3LL * (long long)gridDim.x);
-  long long tile;
-  int mt, nt, ks0, ks1, slot;
+  walk.init(s_active, n_active, p.n_mt, p.k_stages, p.split_counters != nullptr);
+  constexpr int n0 = 0;      // (a single token tile per expert)
+  unsigned tile;
+  int mt, ks0, ks1, slot;
 
   if (warp == 0) {
     // =============================== tile producer (TMA) ===============================
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      while (ok && walk.next<TILE_N>(tile, mt, nt, ks0, ks1, slot)) {
-        const int e = walk.tw.e;
-        const int n0 = nt * TILE_N;
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    while (ok && walk.next(tile, mt, ks0, ks1, slot)) {
+      const int e = walk.e;
 #pragma unroll 1
-        for (int ks = ks0; ks < ks1; ++ks) {
-          if (!ptx::mbar_wait(empty_bar + stage, phase ^ 1)) {
-            atomicExch(&g_status, kProducerEmptyTimeout);
-            ok = false;
-            break;
-          }
-          uint8_t* st = stage_base + stage * C::kStageBytes;
-          const int k_atoms = min(C::kAtoms, p.n_kt - ks * C::kAtoms);
-          const int b_boxes = (k_atoms + 1) / 2;
+      for (int ks = ks0; ks < ks1; ++ks) {
+        if (!ptx::mbar_wait_warp(empty_bar + stage, phase ^ 1)) {
+          atomicExch(&g_status, kProducerEmptyTimeout);
+          ok = false;
+          break;
+        }
+        uint8_t* st = stage_base + stage * C::kStageBytes;
+        const int k_atoms = min(C::kAtoms, p.n_kt - ks * C::kAtoms);
+        const int b_boxes = (k_atoms + 1) / 2;
+        if (ptx::elect_one()) {
           // with the 4-D activation map one copy fetches both 256-K chunks of the stage
           ptx::mbar_arrive_expect_tx(full_bar + stage, C::kABytes + (p.b_4d ? C::kBBoxes : b_boxes) * C::kBBoxBytes);
           ptx::tma_load_3d(st + C::kOffA, &map_a, full_bar + stage, ks * C::kARowBytes, mt * kTileM, e);
@@ -325,96 +310,89 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               ptx::tma_load_3d(st + C::kOffB + b * C::kBBoxBytes, &map_b, full_bar + stage,
                                ks * (STAGE_K / 2) + b * 128, n0, e);
           }
-          if (++stage == p.stages) { stage = 0; phase ^= 1; }
         }
+        __syncwarp();
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
-      if (!ok) {
-        // give copies already in flight time to land before the CTA's shared memory is released
+    }
+    if (!ok) {
+      // give copies already in flight time to land before the CTA's shared memory is released
 #pragma unroll 1
-        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-      }
+      for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     }
     __syncwarp();
   } else if (warp == 1) {
     // =============================== side producer (bulk copies) ===============================
-    // two lanes share every stage (lane 0 the metadata atoms, lane 1 the scale atoms), each with its own
-    // expect-tx arrival
-    if (lane < 2) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      while (ok && walk.next<TILE_N>(tile, mt, nt, ks0, ks1, slot)) {
-        const int e = walk.tw.e;
-        const int n0 = nt * TILE_N;
-        const uint8_t* e_base = p.e_meta + (((long long)e * p.e_k_atoms) * p.e_m_atoms + mt) * 2048;
-        const uint8_t* sfa_base = p.sfa + (((long long)e * p.n_mt + mt) * p.n_kt) * 512;
-        const uint8_t* sfb_base = p.sfb + (((long long)e * p.sfb_rt + (n0 >> 7)) * p.n_kt) * 512;
-        const int sfb_row_atoms = TILE_N > 128 ? min(2, p.sfb_rt - (n0 >> 7)) : 1;
-        for (int ks = ks0; ks < ks1; ++ks) {
-          if (!ptx::mbar_wait(empty_bar + stage, phase ^ 1)) {
-            atomicExch(&g_status, kSideProducerTimeout);
-            ok = false;
-            break;
-          }
-          uint8_t* st = stage_base + stage * C::kStageBytes;
-          const int k_atoms = min(C::kAtoms, p.n_kt - ks * C::kAtoms);
-          const int e_atoms = (k_atoms + 1) / 2;
-          const uint32_t sf_bytes = 512u * k_atoms;
-          const uint8_t* sfa_src = sfa_base + (long long)ks * C::kAtoms * 512;
-          if (lane == 0) {
-            ptx::mbar_arrive_expect_tx(full_bar + stage, e_atoms * 2048);
-            for (int ea = 0; ea < e_atoms; ++ea)
-              ptx::bulk_load(st + C::kOffE + ea * 2048,
-                             e_base + (long long)(ks * C::kEAtoms + ea) * p.e_m_atoms * 2048, 2048,
-                             full_bar + stage);
-          } else {
-            ptx::mbar_arrive_expect_tx(full_bar + stage, sf_bytes * (1 + sfb_row_atoms));
-            ptx::bulk_load(st + C::kOffSfa, sfa_src, sf_bytes, full_bar + stage);
-            for (int ra = 0; ra < sfb_row_atoms; ++ra)
-              ptx::bulk_load(st + C::kOffSfb + ra * C::kSfaBytes,
-                             sfb_base + ((long long)ra * p.n_kt + ks * C::kAtoms) * 512, sf_bytes,
-                             full_bar + stage);
-          }
-          if (++stage == p.stages) { stage = 0; phase ^= 1; }
-        }
-      }
-      if (!ok) {
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    while (ok && walk.next(tile, mt, ks0, ks1, slot)) {
+      const int e = walk.e;
+      const uint8_t* e_base = p.e_meta + (((long long)e * p.e_k_atoms) * p.e_m_atoms + mt) * 2048;
+      const uint8_t* sfa_base = p.sfa + (((long long)e * p.n_mt + mt) * p.n_kt) * 512;
+      const uint8_t* sfb_base = p.sfb + (((long long)e * p.sfb_rt + (n0 >> 7)) * p.n_kt) * 512;
+      const int sfb_row_atoms = TILE_N > 128 ? min(2, p.sfb_rt - (n0 >> 7)) : 1;
 #pragma unroll 1
-        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+      for (int ks = ks0; ks < ks1; ++ks) {
+        if (!ptx::mbar_wait_warp(empty_bar + stage, phase ^ 1)) {
+          atomicExch(&g_status, kSideProducerTimeout);
+          ok = false;
+          break;
+        }
+        uint8_t* st = stage_base + stage * C::kStageBytes;
+        const int k_atoms = min(C::kAtoms, p.n_kt - ks * C::kAtoms);
+        const int e_atoms = (k_atoms + 1) / 2;
+        const uint32_t sf_bytes = 512u * k_atoms;
+        if (ptx::elect_one()) {
+          ptx::mbar_arrive_expect_tx(full_bar + stage, e_atoms * 2048 + sf_bytes * (1 + sfb_row_atoms));
+          for (int ea = 0; ea < e_atoms; ++ea)
+            ptx::bulk_load(st + C::kOffE + ea * 2048,
+                           e_base + (long long)(ks * C::kEAtoms + ea) * p.e_m_atoms * 2048, 2048, full_bar + stage);
+          ptx::bulk_load(st + C::kOffSfa, sfa_base + (long long)ks * C::kAtoms * 512, sf_bytes, full_bar + stage);
+          for (int ra = 0; ra < sfb_row_atoms; ++ra)
+            ptx::bulk_load(st + C::kOffSfb + ra * C::kSfaBytes,
+                           sfb_base + ((long long)ra * p.n_kt + ks * C::kAtoms) * 512, sf_bytes, full_bar + stage);
+        }
+        __syncwarp();
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
+    }
+    if (!ok) {
+#pragma unroll 1
+      for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     }
     __syncwarp();
   } else if (warp < 2 + ISSUERS) {
     // =============================== MMA issuers ===============================
-    if (lane == 0) {
-      const int issuer = warp - 2;
-      constexpr int kPer = C::kAtomsPerIssuer;
-      const int ka0 = issuer * kPer;               // this issuer's K-blocks of a stage: [ka0, ka0 + kPer)
-      constexpr uint32_t idesc = ptx::mma_sp_nvf4_idesc(TILE_N);
-      const uint32_t e_cols = tmem_base + kColE + issuer * C::kEColsPerIssuer;
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
-      bool ok = true;
-      while (ok && walk.next<TILE_N>(tile, mt, nt, ks0, ks1, slot)) {
-        if (!ptx::mbar_wait(acc_empty + acc, acc_phase ^ 1)) {
-          atomicExch(&g_status, kMmaAccTimeout);
+    const int issuer = warp - 2;
+    constexpr int kPer = C::kAtomsPerIssuer;
+    const int ka0 = issuer * kPer;               // this issuer's K-blocks of a stage: [ka0, ka0 + kPer)
+    constexpr uint32_t idesc = ptx::mma_sp_nvf4_idesc(TILE_N);
+    const uint32_t e_cols = tmem_base + kColE + issuer * C::kEColsPerIssuer;
+    int stage = 0, acc = 0;
+    uint32_t phase = 0, acc_phase = 0;
+    bool ok = true;
+    while (ok && walk.next(tile, mt, ks0, ks1, slot)) {
+      if (!ptx::mbar_wait_warp(acc_empty + acc, acc_phase ^ 1)) {
+        atomicExch(&g_status, kMmaAccTimeout);
+        break;
+      }
+      ptx::tc_fence_after();
+      const uint32_t d_tmem = tmem_base + (acc * ISSUERS + issuer) * TILE_N;
+      // (the MMA faults on an odd scale column, which is why 16- and 32-wide tiles exist only for problems with a
+      // single token tile: offset 0)
+      const uint32_t sfb_col = tmem_base + kColSfb;
+#pragma unroll 1
+      for (int ks = ks0; ks < ks1; ++ks) {
+        if (!ptx::mbar_wait_warp(full_bar + stage, phase)) {
+          atomicExch(&g_status, kMmaFullTimeout);
+          ok = false;
           break;
         }
         ptx::tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (acc * ISSUERS + issuer) * TILE_N;
-        // The scales of a 64-wide tile's rows sit 0 or 2 columns into the 128-row atom.  The MMA
-        // faults (misaligned address) on an odd column offset, which is why 16- and 32-wide tiles
-        // exist only for problems with a single token tile (offset 0).
-        const uint32_t sfb_col = tmem_base + kColSfb + (TILE_N < 128 ? ((nt * TILE_N) & 127) >> 5 : 0);
-        for (int ks = ks0; ks < ks1; ++ks) {
-          if (!ptx::mbar_wait(full_bar + stage, phase)) {
-            atomicExch(&g_status, kMmaFullTimeout);
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
-          const uint32_t st = ptx::smem_u32(stage_base + stage * C::kStageBytes);
-          const int k_atoms = min(C::kAtoms, p.n_kt - ks * C::kAtoms);
+        const uint32_t st = ptx::smem_u32(stage_base + stage * C::kStageBytes);
+        const int k_atoms = min(C::kAtoms, p.n_kt - ks * C::kAtoms);
+        if (ptx::elect_one()) {
           if (ka0 < k_atoms) {
             // metadata atoms covering this issuer's K-blocks, into its private columns
 #pragma unroll
@@ -451,13 +429,14 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
                                   tmem_base + kColSfa + ka * 4, sfb_col + ka * C::kSfbColsPerAtom, e_tmem);
             }
           }
-          ptx::tc_commit(empty_bar + stage);   // stage reusable once every issuer's MMAs and copies retire
-          if (++stage == p.stages) { stage = 0; phase ^= 1; }
+          ptx::tc_commit(empty_bar + stage);     // stage reusable once every issuer's MMAs and copies retire
+          if (ks + 1 == ks1) ptx::tc_commit(acc_full + acc);      // this issuer's partial accumulator is complete
         }
-        if (!ok) break;
-        ptx::tc_commit(acc_full + acc);        // this issuer's partial accumulator is complete
-        if (++acc == C::kAccStages) { acc = 0; acc_phase ^= 1; }
+        __syncwarp();
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
+      if (!ok) break;
+      if (++acc == C::kAccStages) { acc = 0; acc_phase ^= 1; }
     }
     __syncwarp();
   } else {
@@ -501,16 +480,16 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       }
     }
     int* s_last = reinterpret_cast<int*>(tmem_slot + 1);     // "this CTA arrived last at the tile", told to all epilogue threads
-    while (walk.next<TILE_N>(tile, mt, nt, ks0, ks1, slot)) {
-      const int e = walk.tw.e;
+    while (walk.next(tile, mt, ks0, ks1, slot)) {
+      const int e = walk.e;
       const int cnt = s_counts[e];
+      const float alpha = p.alphas[e];           // (in flight while the warp waits)
+      const float gs = kFused ? (p.f_gpe ? p.f_gscale[e] : p.f_gscale[0]) : 0.f;
       if (!ptx::mbar_wait(acc_full + acc, acc_phase)) {
         atomicExch(&g_status, kEpilogueTimeout);
         break;
       }
       ptx::tc_fence_after();
-      const float alpha = p.alphas[e];
-      const int n0 = nt * TILE_N;
       const long long row_e = (long long)e * p.max_n;
       // Issuers whose partial accumulators hold something for this unit.  Every issuer has K-blocks in a full
       // stage; in the (shorter) last stage of a tile the later issuers may have none, and a unit that is just
@@ -545,7 +524,7 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           __threadfence();
           epilogue_bar_sync();
           // the CTAs that share this tile, first to last in K
-          const unsigned t_lo = (unsigned)tile * walk.ksn, t_hi = t_lo + walk.ksn;
+          const unsigned t_lo = tile * walk.ksn, t_hi = t_lo + walk.ksn;
           const unsigned c_first = walk.owner(t_lo), c_last = walk.owner(t_hi - 1);
           const int parts = (int)(c_last - c_first + 1);        // every CTA in between holds stages of the tile
           if (ep_tid == 0) {
@@ -575,54 +554,34 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           __nv_bfloat16 h[kCols];
 #pragma unroll
           for (int i = 0; i < kCols; ++i) h[i] = __float2bfloat16_rn(__fmul_rn(alpha, __uint_as_float(r[i])));
-          // Every lane parks its values; then the gate lane of a feature finishes the even token
-          // columns and the up lane of the same feature the odd ones, each reading its partner's
-          // value from shared memory and leaving the product in the gate's slot.  Loads, math and
-          // stores are kept in separate passes so the 8 or 16 independent chains overlap.
-          const bool is_up = (sub & 1) != 0;
+          // Every lane parks its values; then a thread takes half a block of one token - 16 features - and
+          // everything is in its registers: activation, amax (one exchange with the lane that has the other
+          // half), scale, codes.  (Rows of 272 bytes: eight lanes' 16-byte reads fall in different banks.)
 #pragma unroll
           for (int i = 0; i < kCols; ++i) buf[i * kOutRow + m_local] = h[i];
           epilogue_bar_sync();
-          constexpr int kHalf = kCols / 2;
-          const int par = is_up ? 1 : 0;
-          const int g_row = is_up ? m_local - 32 : m_local;   // the gate's slot, which receives the product
-          __nv_bfloat16* col0 = buf + par * kOutRow + g_row;
-#pragma unroll 1
-          for (int i0 = 0; i0 < kHalf; i0 += 4) {
-            float g[4], u[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              g[i] = __bfloat162float(col0[(i0 + i) * 2 * kOutRow]);
-              u[i] = __bfloat162float(col0[(i0 + i) * 2 * kOutRow + 32]);
-            }
-            __nv_bfloat16 y[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) y[i] = __float2bfloat16_rn(gated_act(g[i], u[i], p.f_act));
-#pragma unroll
-            for (int i = 0; i < 4; ++i) col0[(i0 + i) * 2 * kOutRow] = y[i];
-          }
-          epilogue_bar_sync();
-          if (ep_tid < 64) {
-            const int i = ep_tid & 31, blk = ep_tid >> 5;
-            const int n = n0 + c0 + i;
-            if (i < kCols && n < cnt) {
-              const uint4* src = reinterpret_cast<const uint4*>(buf + i * kOutRow + blk * 64);
-              float f[4][8];
-              float amax = 0.f;
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                unpack8(src[q], f[q]);
-#pragma unroll
-                for (int z = 0; z < 8; ++z) amax = fmaxf(amax, fabsf(f[q][z]));
-              }
+          const int blk = (ep_tid >> 5) & 1, half = lane >> 4;
+          const int t = (lane & 15) + 16 * (ep_tid >> 6);      // this lane's token column
+          const int n = n0 + c0 + t;
+          if (16 * (ep_tid >> 6) < kCols) {                      // uniform over the warp
+            uint32_t y[8];
+            const uint4* gp = reinterpret_cast<const uint4*>(buf + t * kOutRow + blk * 64 + half * 16);
+            const uint4 g0 = gp[0], g1 = gp[1], u0 = gp[4], u1 = gp[5];
+            const uint32_t g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+            const uint32_t u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+            gated_act16(g, u, p.f_act, y);
+            uint32_t m = bf16x2_amax8(y);
+            m = bf16x2_max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+            const float amax = fmaxf(fmaxf(bf16_lo(m), bf16_hi(m)), 0.f);
+            if (n < cnt) {
               uint32_t sf_byte;
               float inv;
-              block_scale(amax, p.f_gpe ? p.f_gscale[e] : p.f_gscale[0], sf_byte, inv);
-              const int kb = mt * 2 + blk;     // 32-feature block of the N-wide output
-              const long long row = (long long)e * p.max_n + n;
-              *reinterpret_cast<uint4*>(p.f_b_out + row * (p.f_n / 2) + kb * 16) =
-                  make_uint4(quant8(f[0], inv), quant8(f[1], inv), quant8(f[2], inv), quant8(f[3], inv));
-              p.f_sfb_out[sf_offset(e, n, kb, p.sfb_rt, p.f_n_kt)] = (uint8_t)sf_byte;
+              block_scale(amax, gs, sf_byte, inv);
+              const int kb = mt * 2 + blk;       // 32-feature block of the N-wide output
+              const long long row = row_e + n;
+              *reinterpret_cast<uint2*>(p.f_b_out + row * (p.f_n / 2) + kb * 16 + half * 8) =
+                  make_uint2(quant8_packed(y[0], y[1], y[2], y[3], inv), quant8_packed(y[4], y[5], y[6], y[7], inv));
+              if (half == 0) p.f_sfb_out[sf_offset(e, n, kb, p.sfb_rt, p.f_n_kt)] = (uint8_t)sf_byte;
             }
           }
           ++chunk;
@@ -836,7 +795,7 @@ int launch_narrow_impl(const CUtensorMap& map_a, const CUtensorMap& map_b, const
   using C = Cfg<TILE_N, STAGE_K, ISSUERS>;
   Params p = p_in;
   p.stages = C::kStages;
-  const size_t smem = 1024 + (size_t)C::kStages * C::kStageBytes + kOutStageBytes + 256 + 4 * (size_t)p.E;
+  const size_t smem = 1024 + (size_t)C::kStages * C::kStageBytes + kOutStageBytes + 256 + 6 * (size_t)p.E;
   static_assert(kOutStageBytes % 16 == 0, "barrier block must stay aligned");
   static_assert(8 * (2 * C::kStages + 2 * C::kAccStages) + 16 <= 256, "barrier block overflows its slot");
   static KernelSetup setup;
@@ -1011,7 +970,7 @@ struct FusedArgs {
   uint8_t* sfb_out = nullptr;
   const float* gscale = nullptr;
   int gpe = 0;
-  GatedAct act{PNV_ACT_SILU, 1.f, -1.f, 0};
+  GatedAct act{};
 };
 
 // The tile variants of the fused op, by the reference's names (csrc/sm100/tactics.cu:52-57).
@@ -1060,7 +1019,7 @@ int group_mm_common(void* out, const int32_t* row_map, const RowParts* out_parts
   p.row_map = row_map;
   p.out_parts = out_parts ? *out_parts : RowParts{};
   p.f_b_out = nullptr; p.f_sfb_out = nullptr; p.f_gscale = nullptr; p.f_gpe = 0; p.f_n = 0; p.f_n_kt = 0;
-  p.f_act = GatedAct{PNV_ACT_SILU, 1.f, -1.f, 0};
+  p.f_act = GatedAct{};
   if (fused != nullptr) {
     p.f_b_out = fused->b_out; p.f_sfb_out = fused->sfb_out; p.f_gscale = fused->gscale; p.f_gpe = fused->gpe;
     p.f_n = features / 2; p.f_n_kt = sf_k_atoms(features / 2); p.f_act = fused->act;
