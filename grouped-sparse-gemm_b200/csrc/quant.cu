@@ -406,10 +406,10 @@ static bool g_silu_short = true;
 
 int make_gated_act(int act_kind, float beta, float linear_beta, GatedAct& out) {
   if (act_kind == PNV_ACT_SILU) {
-    out = GatedAct{PNV_ACT_SILU, 1.0f, -1.0f, g_silu_short ? 0 : 1};
+    out = GatedAct{PNV_ACT_SILU, 1.0f, -1.0f, 1.0f, -1.0f, g_silu_short ? 0 : 1};
   } else if (act_kind == PNV_ACT_SITU) {
     PNV_REQUIRE(beta > 0, "situ: beta must be positive, got %g", (double)beta);
-    out = GatedAct{PNV_ACT_SITU, beta, linear_beta, 0};
+    out = GatedAct{PNV_ACT_SITU, beta, linear_beta, 1.0f / beta, 1.0f / linear_beta, 0};
   } else {
     return fail(PNV_ERR_INVALID_ARGUMENT, "activation must be 'silu' or 'situ', got kind %d", act_kind);
   }
@@ -425,7 +425,7 @@ extern "C" int pnv_quant_act(const void* x, const float* gscale, int gscale_per_
                              uint8_t* sfb, int sm_count, pnv_stream_t stream) {
   if (int rc = check_common(x, gscale, counts, experts, max_n, k, b_act, sfb, "K")) return rc;
   long long lines = sf_numel(max_n, k, experts) / 16;
-  GatedAct act{PNV_ACT_SILU, 1.f, -1.f, 0};
+  GatedAct act{};
   PNV_CUDA(launch_pdl(quant_lines_kernel<kPlain>, dim3(grid_for(lines, sm_count)), dim3(kThreads), 0,
                       (cudaStream_t)stream, pdl_enabled(), (const __nv_bfloat16*)x, gscale,
                       gscale_per_expert, counts, experts, max_n, k, 0, act, b_act, sfb));
