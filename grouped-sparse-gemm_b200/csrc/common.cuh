@@ -134,18 +134,16 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 
 // ---- numeric conversions ------------------------------------------------------------------------
 
-// Two floats -> two e2m1 nibbles (lo in bits 0-3), round-to-nearest-even, saturating to +-6.
-__device__ __forceinline__ uint32_t cvt_e2m1x2(float lo, float hi) {
-  uint32_t r;
-  asm("{\n\t.reg .b8 b;\n\tcvt.rn.satfinite.e2m1x2.f32 b, %2, %1;\n\tcvt.u32.u8 %0, b;\n\t}"
-      : "=r"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-
-// Eight floats -> one 32-bit word of e2m1 nibbles, element j in nibble j.
+// Eight floats -> one 32-bit word of e2m1 nibbles, element j in nibble j (round-to-nearest-even, saturating to +-6).  (One
+// statement: the four bytes are packed by a vector move, where separate conversions cost a widening, a shift and an or each.)
 __device__ __forceinline__ uint32_t cvt_e2m1x8(const float (&v)[8]) {
-  return cvt_e2m1x2(v[0], v[1]) | (cvt_e2m1x2(v[2], v[3]) << 8) | (cvt_e2m1x2(v[4], v[5]) << 16) |
-         (cvt_e2m1x2(v[6], v[7]) << 24);
+  uint32_t r;
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\tcvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\tcvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+      : "=r"(r) : "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]));
+  return r;
 }
 
 // float -> UE4M3 byte, round-to-nearest-even, saturating to 448.
@@ -175,17 +173,10 @@ __device__ __forceinline__ void block_scale(float amax, float g, uint32_t& sf_by
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }
 
-// Eight bf16 (one 128-bit word) -> floats, and eight floats -> one word of e2m1 codes after scaling.
+// Eight bf16 (one 128-bit word) -> floats.
 __device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
   f[0] = bf16_lo(v.x); f[1] = bf16_hi(v.x); f[2] = bf16_lo(v.y); f[3] = bf16_hi(v.y);
   f[4] = bf16_lo(v.z); f[5] = bf16_hi(v.z); f[6] = bf16_lo(v.w); f[7] = bf16_hi(v.w);
-}
-
-__device__ __forceinline__ uint32_t quant8(const float (&f)[8], float inv) {
-  float s[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) s[i] = __fmul_rn(f[i], inv);
-  return cvt_e2m1x8(s);
 }
 
 // The gated activation applied between the two expert GEMMs, with the rounding chain of the
@@ -279,10 +270,16 @@ __device__ __forceinline__ uint32_t bf16x2_amax8(const uint32_t (&y)[8]) {
   for (int i = 1; i < 8; ++i) m = bf16x2_max(m, y[i] & 0x7FFF7FFFu);
   return m;
 }
-// quant8 for values that sit in four such registers.
+// Eight bf16 in four registers -> one word of e2m1 codes after scaling by inv (two products to an instruction, each rounded
+// as on its own).
 __device__ __forceinline__ uint32_t quant8_packed(uint32_t a, uint32_t b, uint32_t c, uint32_t d, float inv) {
-  const float f[8] = {bf16_lo(a), bf16_hi(a), bf16_lo(b), bf16_hi(b), bf16_lo(c), bf16_hi(c), bf16_lo(d), bf16_hi(d)};
-  return quant8(f, inv);
+  const uint32_t w[4] = {a, b, c, d};
+  float v[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %4};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(v[2 * i]), "=f"(v[2 * i + 1]) : "f"(bf16_lo(w[i])), "f"(bf16_hi(w[i])), "f"(inv));
+  return cvt_e2m1x8(v);
 }
 // The gated activation of 16 neighbouring features.  silu(g) is a bf16 number and the product of two bf16 numbers is
 // exact in float, so one packed bf16 multiplication rounds like the float product rounded to bf16.

@@ -1,17 +1,20 @@
 // Activation quantizers: bf16 -> e2m1 codes + one UE4M3 scale per 32 elements, written straight
 // into the grouped GEMM's B-operand layouts (row-major codes, swizzled scale atoms).
 //
-// quant_act and silu_mul_quant_act walk the *scale buffer*: one warp owns one 16-byte line of a
-// scale atom, i.e. the 4 rows {r, r+32, r+64, r+96} x 4 K-blocks whose scales share that line.
-// The warp quantizes the (up to) 4 x 128 elements behind it with 128-bit loads, reduces each
-// block's amax with one shuffle, and writes the line once -- quantized scales where a row is live,
-// the benign byte 0x38 everywhere else -- so the scale buffer is fully defined without a separate
-// fill pass and without byte-sized stores.  Lines whose rows are all past the expert's token
-// count cost one 16-byte store.
+// quant_act, silu_mul_quant_act and scatter_quant_act_planned share one kernel.  Its units are the live rows (r < counts[e])
+// of the batched operand, found through a prefix sum of counts that every block makes for itself, so that skewed or mostly
+// empty capacities cost nothing: a warp takes a row, or a piece of one where there are fewer rows than warps, 32 K-blocks
+// at a time with one whole block per lane (64 bytes in, or 128 with gate and up; 16 bytes of codes out; the scale step,
+// with its two IEEE divisions, once per block).  The bytes of the scale buffer that no live row writes become 0x38 in the
+// same kernel, a 16-byte line per thread.
+// Bound: HBM for plain rows (131072 rows of 2048: 118 us, 687 MB), issue slots (0.68 of them used) and L2 for gathered
+// ones (102 us; 150 MB written, the rows read from L2 eight times over), the special-function unit and issue for SiTU.
+// Loads are 32 bytes a lane where the input is aligned to that: 16-byte loads at a stride of 64 bytes take twice the
+// passes through L1.  Before, a warp per 16-byte line of the scale buffer, dead lines included: 466 us for 32768 live
+// rows of 3072 (SiTU) in a capacity of 524288, now 172; the gather of those rows 82 us, now 40.
 //
-// scatter_quant_act is driven by a routing list instead (source token -> destination row), so its
-// scale buffer is pre-filled with a memset node and each warp quantizes 256 elements of one routed
-// row.
+// scatter_quant_act is driven by a flat routing list instead (source token -> destination row), so its scale buffer is
+// pre-filled with a memset node.
 #include "common.cuh"
 
 namespace pnv {
@@ -20,160 +23,68 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kWarpsPerBlock = kThreads / 32;
 
-// Gather the 16 scale bytes of a line from the lanes that own them (lane g*8 + 2*kq holds the
-// byte of row group g, K-block kq) and store them as four 32-bit words.
-__device__ __forceinline__ void store_sf_line(uint8_t* line, uint32_t my_byte, int lane) {
-  int g8 = lane & ~7;
-  uint32_t w = __shfl_sync(0xffffffffu, my_byte, g8 + 0) |
-               (__shfl_sync(0xffffffffu, my_byte, g8 + 2) << 8) |
-               (__shfl_sync(0xffffffffu, my_byte, g8 + 4) << 16) |
-               (__shfl_sync(0xffffffffu, my_byte, g8 + 6) << 24);
-  if ((lane & 7) == 0) *reinterpret_cast<uint32_t*>(line + (lane >> 3) * 4) = w;
-}
-
-// Where a live row's values come from.
-//   kPlain   x is [E, max_n, K]
-//   kGated   x is [E, max_n, 2K] holding gate and up; the gated activation is applied first
-enum LineSource : int { kPlain = 0, kGated = 1 };
-
-template <int kSrc>
-__global__ void __launch_bounds__(kThreads)
-quant_lines_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gscale,
-                   int gscale_per_expert, const int* __restrict__ counts, int E, int max_n, int K,
-                   int interleaved, GatedAct act, uint8_t* __restrict__ b_act,
-                   uint8_t* __restrict__ sfb) {
-  pdl_wait();
-  pdl_launch_dependents();
-  const int KB = K / kSfBlock;
-  const int n_rt = sf_row_atoms(max_n);
-  const int n_kt = sf_k_atoms(K);
-  // line arithmetic in 32 bits (the host checks the line count): 64-bit divisions per line once
-  // cost more instructions than the quantization itself
-  const unsigned lines = (unsigned)E * n_rt * n_kt * 32u;
-  const int lane = threadIdx.x & 31;
-  const int g = lane >> 3;          // row group inside the atom: rows rr + 32 g
-  const int j = lane & 7;           // 16-element piece of the 128-element segment
-  const unsigned warp0 = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  const unsigned nwarps = gridDim.x * kWarpsPerBlock;
-  const uint32_t benign4 = kBenignSf * 0x01010101u;
-
-  for (unsigned c = warp0; c < lines; c += nwarps) {
-    const int rr = (int)(c & 31);
-    const unsigned a = c >> 5;
-    const unsigned a_kt = a / (unsigned)n_kt;
-    const int kt = (int)(a - a_kt * n_kt);
-    const int e = (int)(a_kt / (unsigned)n_rt);
-    const int rt = (int)(a_kt - (unsigned)e * n_rt);
-    const int cnt = min(counts[e], max_n);
-    uint8_t* line = sfb + (long long)c * 16;
-    if (rt * 128 + rr >= cnt) {   // no live row behind this line
-      if (lane == 0) *reinterpret_cast<uint4*>(line) = make_uint4(benign4, benign4, benign4, benign4);
-      continue;
-    }
-    const int r = rt * 128 + rr + 32 * g;
-    const int kb = kt * 4 + (j >> 1);
-    const bool live = (r < cnt) && (kb < KB);
-    const int k0 = kb * kSfBlock + (j & 1) * 16;
-    uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
-    float f0[8], f1[8];
-    if (live) {
-      const long long row = (long long)e * max_n + r;
-      if (kSrc == kPlain) {
-        const uint4* p = reinterpret_cast<const uint4*>(x + row * K + k0);
-        v0 = __ldg(p);
-        v1 = __ldg(p + 1);
-        unpack8(v0, f0);
-        unpack8(v1, f1);
-      } else {
-        const __nv_bfloat16* base = x + row * (2LL * K);
-        const int gate_off = interleaved ? kb * 64 + (j & 1) * 16 : k0;
-        const int up_off = interleaved ? gate_off + 32 : K + k0;
-        const uint4* pg = reinterpret_cast<const uint4*>(base + gate_off);
-        const uint4* pu = reinterpret_cast<const uint4*>(base + up_off);
-        uint4 g0 = __ldg(pg), g1 = __ldg(pg + 1), u0 = __ldg(pu), u1 = __ldg(pu + 1);
-        float ga[8], ua[8];
-        unpack8(g0, ga); unpack8(u0, ua);
-        float gb[8], ub[8];
-        unpack8(g1, gb); unpack8(u1, ub);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) f0[i] = gated_act(ga[i], ua[i], act);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) f1[i] = gated_act(gb[i], ub[i], act);
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) { f0[i] = 0.f; f1[i] = 0.f; }
-    }
-    float amax = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fmaxf(fabsf(f0[i]), fabsf(f1[i])));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-    uint32_t sf_byte = kBenignSf;
-    if (live) {
-      const float gs = gscale_per_expert ? gscale[e] : gscale[0];
-      float inv;
-      block_scale(amax, gs, sf_byte, inv);
-      uint2 codes = make_uint2(quant8(f0, inv), quant8(f1, inv));
-      const long long row = (long long)e * max_n + r;
-      *reinterpret_cast<uint2*>(b_act + row * (K / 2) + k0 / 2) = codes;
-    }
-    store_sf_line(line, sf_byte, lane);
-  }
-}
-
 // Four adjacent lanes hold the scale bytes of four consecutive K-blocks; lane 4j returns their word.
 __device__ __forceinline__ uint32_t gather_sf_word(uint32_t my_byte) {
   return my_byte | (__shfl_down_sync(0xffffffffu, my_byte, 1) << 8) |
          (__shfl_down_sync(0xffffffffu, my_byte, 2) << 16) | (__shfl_down_sync(0xffffffffu, my_byte, 3) << 24);
 }
 
-// One 32-element block in one lane: 64 bytes in, amax, scale, 16 bytes of codes.  Doing the whole
-// block in a lane runs the scale step (two IEEE divisions, two format conversions) once per block
-// instead of once per 8 elements, which is what bounds these kernels on B200.
+// One 32-element block in one lane: 64 bytes in, two bf16 to a register.  `wide`: the source is 32-byte aligned.
 struct BlockRegs {
-  float f[4][8];
+  uint32_t lo[8], hi[8];
 };
-__device__ __forceinline__ void load_block(const uint4* src, BlockRegs& b) {
-  uint4 v0 = __ldg(src), v1 = __ldg(src + 1), v2 = __ldg(src + 2), v3 = __ldg(src + 3);
-  unpack8(v0, b.f[0]); unpack8(v1, b.f[1]); unpack8(v2, b.f[2]); unpack8(v3, b.f[3]);
+__device__ __forceinline__ void load32(const uint8_t* src, bool wide, uint32_t (&w)[8]) {
+  if (wide) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(src));
+  } else {
+    const uint4 v0 = __ldg(reinterpret_cast<const uint4*>(src)), v1 = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+    w[0] = v0.x; w[1] = v0.y; w[2] = v0.z; w[3] = v0.w;
+    w[4] = v1.x; w[5] = v1.y; w[6] = v1.z; w[7] = v1.w;
+  }
+}
+__device__ __forceinline__ void load_block(const uint8_t* src, bool wide, BlockRegs& b) {
+  load32(src, wide, b.lo);
+  load32(src + 32, wide, b.hi);
 }
 __device__ __forceinline__ float block_amax(const BlockRegs& b) {
-  float m = 0.f;
-#pragma unroll
-  for (int q = 0; q < 4; ++q)
-#pragma unroll
-    for (int z = 0; z < 8; ++z) m = fmaxf(m, fabsf(b.f[q][z]));
-  return m;
+  const uint32_t m = bf16x2_max(bf16x2_amax8(b.lo), bf16x2_amax8(b.hi));
+  return fmaxf(fmaxf(bf16_lo(m), bf16_hi(m)), 0.f);       // (a NaN counts as nothing)
 }
 __device__ __forceinline__ uint4 block_codes(const BlockRegs& b, float inv) {
-  return make_uint4(quant8(b.f[0], inv), quant8(b.f[1], inv), quant8(b.f[2], inv), quant8(b.f[3], inv));
+  return make_uint4(quant8_packed(b.lo[0], b.lo[1], b.lo[2], b.lo[3], inv), quant8_packed(b.lo[4], b.lo[5], b.lo[6], b.lo[7], inv),
+                    quant8_packed(b.hi[0], b.hi[1], b.hi[2], b.hi[3], inv), quant8_packed(b.hi[4], b.hi[5], b.hi[6], b.hi[7], inv));
+}
+// Every value times the bf16 weight w, rounded to bf16 (the product of two bf16 numbers is exact in float, so the packed
+// multiplication rounds like the float product rounded to bf16).
+__device__ __forceinline__ void block_weight(BlockRegs& b, float w) {
+  const __nv_bfloat162 w2 = __float2bfloat162_rn(w);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    b.lo[i] = as_u32(__hmul2(as_bf162(b.lo[i]), w2));
+    b.hi[i] = as_u32(__hmul2(as_bf162(b.hi[i]), w2));
+  }
 }
 
-// One routed row by one warp: 32 K-blocks (1024 elements) at a time, one block per lane; a row's four scales
-// of one 128-K group are one aligned word of the swizzled layout.  `w` is the (already bf16-rounded) router
-// weight when `weighted`.
-__device__ __forceinline__ void quantize_routed_row(const uint4* __restrict__ src, uint4* __restrict__ dst,
-                                                    uint8_t* __restrict__ sf_row, int KB, float gs, bool weighted,
-                                                    float w, int lane) {
-  for (int kb0 = 0; kb0 < KB; kb0 += 32) {
-    const int kb = kb0 + lane;
-    uint32_t sf_byte = kBenignSf;   // blocks past K keep the benign byte in the layout's slop
-    if (kb < KB) {
-      BlockRegs b;
-      load_block(src + kb * 4, b);
-      if (weighted) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-#pragma unroll
-          for (int z = 0; z < 8; ++z) b.f[q][z] = __bfloat162float(__float2bfloat16_rn(__fmul_rn(b.f[q][z], w)));
-      }
-      float inv;
-      block_scale(block_amax(b), gs, sf_byte, inv);
-      dst[kb] = block_codes(b, inv);
-    }
-    const uint32_t word = gather_sf_word(sf_byte);
-    if ((lane & 3) == 0 && kb < KB) *reinterpret_cast<uint32_t*>(sf_row + (kb >> 2) * 512) = word;
+// Where a row's values come from.
+//   kPlain   the row itself, x is [E, cap, K]
+//   kGated   x is [E, cap, 2K] holding gate and up; the gated activation is applied first
+//   kGather  row src_tok[slot] of x [T, K], optionally times the router weight of routing src_route[slot]
+enum RowSource : int { kPlain = 0, kGated = 1, kGather = 2 };
+
+// 32 K-blocks from kb0 on, one per lane in b, are scaled, rounded and stored; a row's four scales of one 128-K group are one
+// aligned word of the swizzled layout.  KB: the blocks of the whole row.
+__device__ __forceinline__ void finish_blocks(const BlockRegs& b, int kb0, int KB, float gs, uint4* __restrict__ dst,
+                                              uint8_t* __restrict__ sf_row, int lane) {
+  const int kb = kb0 + lane;
+  uint32_t sf_byte = kBenignSf;   // blocks past K keep the benign byte in the layout's slop
+  if (kb < KB) {
+    float inv;
+    block_scale(block_amax(b), gs, sf_byte, inv);
+    dst[kb] = block_codes(b, inv);
   }
+  const uint32_t word = gather_sf_word(sf_byte);
+  if ((lane & 3) == 0 && kb < KB) *reinterpret_cast<uint32_t*>(sf_row + (kb >> 2) * 512) = word;
 }
 
 // scatter_quant_act: one warp per routing of the flat plan.
@@ -188,6 +99,7 @@ scatter_quant_kernel(const __nv_bfloat16* __restrict__ a1, const long long* __re
   const int n_rt = sf_row_atoms(cap);
   const int n_kt = sf_k_atoms(K);
   const long long trash = (long long)E * cap;
+  const bool wide = (reinterpret_cast<uintptr_t>(a1) & 31) == 0;
   const int lane = threadIdx.x & 31;
   const unsigned warp0 = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const unsigned nwarps = gridDim.x * kWarpsPerBlock;
@@ -199,86 +111,250 @@ scatter_quant_kernel(const __nv_bfloat16* __restrict__ a1, const long long* __re
     const float gs = gscale_per_expert ? gscale[e] : gscale[0];
     const bool weighted = topk_w != nullptr;
     const float w = weighted ? __bfloat162float(__float2bfloat16_rn(topk_w[i])) : 1.f;
-    quantize_routed_row(reinterpret_cast<const uint4*>(a1 + flat_tok[i] * K),
-                        reinterpret_cast<uint4*>(b_act + dest * (K / 2)), sfb + sf_offset(e, r, 0, n_rt, n_kt), KB, gs,
-                        weighted, w, lane);
+    const uint8_t* src = reinterpret_cast<const uint8_t*>(a1 + flat_tok[i] * K);
+    for (int kb0 = 0; kb0 < KB; kb0 += 32) {
+      BlockRegs b;
+      if (kb0 + lane < KB) load_block(src + 64LL * (kb0 + lane), wide, b);
+      if (weighted) block_weight(b, w);
+      finish_blocks(b, kb0, KB, gs, reinterpret_cast<uint4*>(b_act + dest * (K / 2)), sfb + sf_offset(e, r, 0, n_rt, n_kt), lane);
+    }
   }
 }
 
-// scatter_quant_act_planned: one warp per row slot (e, r) of the batched operand; slots at or past counts[e] are
-// skipped (their scales keep the benign fill laid down before the launch).
-__global__ void __launch_bounds__(kThreads)
-scatter_planned_rows_kernel(const __nv_bfloat16* __restrict__ a1, const int* __restrict__ src_tok,
-                            const int* __restrict__ src_route, const float* __restrict__ topk_w,
-                            const float* __restrict__ gscale, int gscale_per_expert, const int* __restrict__ counts,
-                            int K, int E, int cap, uint8_t* __restrict__ b_act, uint8_t* __restrict__ sfb) {
+// Every byte of a scale buffer that no live row (r < counts[e]) writes becomes 0x38: whole 16-byte lines behind which
+// no row is live, single words of the others.  (K-block slop of a live row is part of the words that row writes.)  The
+// kernels that place rows do this themselves, each thread a share of the lines: as a memset in front of them it was a
+// launch of its own and kept them from starting while their predecessor drains.
+__device__ __forceinline__ void benign_fill_dead(const int* __restrict__ counts, int E, int cap, int n_rt, int n_kt,
+                                                 uint8_t* __restrict__ sfb) {
+  const uint32_t w4 = kBenignSf * 0x01010101u;
+  const unsigned lines = (unsigned)E * n_rt * n_kt * 32u;
+  for (unsigned c = blockIdx.x * kThreads + threadIdx.x; c < lines; c += gridDim.x * kThreads) {
+    const unsigned a_kt = (c >> 5) / (unsigned)n_kt;
+    const unsigned e = a_kt / (unsigned)n_rt;
+    const int r0 = (int)(a_kt - e * (unsigned)n_rt) * 128 + (int)(c & 31);
+    const int cnt = min(counts[e], cap);
+    uint8_t* line = sfb + (long long)c * 16;
+    if (r0 >= cnt) {
+      *reinterpret_cast<uint4*>(line) = make_uint4(w4, w4, w4, w4);
+    } else {
+#pragma unroll
+      for (int g = 1; g < 4; ++g)
+        if (r0 + 32 * g >= cnt) *reinterpret_cast<uint32_t*>(line + 4 * g) = w4;
+    }
+  }
+}
+
+// The live rows of a batched operand, numbered expert after expert.  make() builds the prefix sums of the clamped
+// counts - up to 32 experts every warp in its own registers, without a barrier; up to kMaxPrefixExperts the block in
+// shared memory - and find() turns a row's number into its slot.  With more experts there are no prefix sums: every slot is
+// a row and the dead ones are skipped.  All lanes of a warp ask for the same row.
+constexpr int kMaxPrefixExperts = 8192;
+struct LiveRows {
+  const int* counts;
+  int E, cap;
+  int* prefix;           // shared memory, [E + 1]
+  int lane_first;        // up to 32 experts: first row of expert `lane` (INT_MAX past the last)
+  unsigned total;
+  __device__ __forceinline__ void make(const int* counts_, int E_, int cap_, int* smem) {
+    counts = counts_; E = E_; cap = cap_; prefix = smem; lane_first = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (E > kMaxPrefixExperts) { total = (unsigned)E * (unsigned)cap; return; }
+    if (E <= 32) {
+      const int c = lane < E ? max(0, min(counts[lane], cap)) : 0;
+      int v = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      lane_first = lane < E ? v - c : 0x7FFFFFFF;
+      total = (unsigned)__shfl_sync(0xffffffffu, v, 31);
+      return;
+    }
+    __shared__ int s_warp[kWarpsPerBlock];
+    int carry = 0;
+    for (int e0 = 0; e0 < E; e0 += kThreads) {
+      const int e = e0 + (int)threadIdx.x;
+      int v = e < E ? max(0, min(counts[e], cap)) : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      if (lane == 31) s_warp[warp] = v;
+      __syncthreads();
+      int before = carry, sum = 0;
+#pragma unroll
+      for (int i = 0; i < kWarpsPerBlock; ++i) {
+        if (i < warp) before += s_warp[i];
+        sum += s_warp[i];
+      }
+      if (e < E) smem[e + 1] = before + v;
+      carry += sum;
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) smem[0] = 0;
+    __syncthreads();
+    total = (unsigned)carry;
+  }
+  // row number j < total -> expert and row of the expert; false for a dead slot (only without prefix sums)
+  __device__ __forceinline__ bool find(unsigned j, int& e, int& r) const {
+    if (E <= 32) {       // the last expert whose first row is at or before j
+      e = 31 - __clz(__ballot_sync(0xffffffffu, (unsigned)lane_first <= j));
+      r = (int)j - __shfl_sync(0xffffffffu, lane_first, e);
+      return true;
+    }
+    if (E > kMaxPrefixExperts) {
+      e = (int)(j / (unsigned)cap);
+      r = (int)(j - (unsigned)e * (unsigned)cap);
+      return r < counts[e];
+    }
+    int lo = 0, hi = E - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if ((unsigned)prefix[mid] <= j) lo = mid;
+      else hi = mid - 1;
+    }
+    e = lo;
+    r = (int)j - prefix[lo];
+    return true;
+  }
+};
+size_t live_rows_smem(int E) { return E <= 32 || E > kMaxPrefixExperts ? 0 : sizeof(int) * (size_t)(E + 1); }
+
+struct RowsArgs {
+  const __nv_bfloat16* x;
+  const int* src_tok;
+  const int* src_route;
+  const float* topk_w;
+  const float* gscale;
+  const int* counts;
+  uint8_t* b_act;
+  uint8_t* sfb;
+  GatedAct act;
+  int gscale_per_expert, E, cap, K, interleaved;
+};
+
+// Blocks per SM: four hold 64 registers a thread; five or six spill (6 to 17 % slower with the activation), three with the
+// next step's loads ahead of the arithmetic are 15 % slower.  The grid is one wave of them.
+constexpr int kBatchedBlocks = 4;
+
+template <int kSrc>
+__global__ void __launch_bounds__(kThreads, kBatchedBlocks)
+quant_batched_kernel(const RowsArgs a) {
+  extern __shared__ int s_prefix[];
   pdl_wait();
   pdl_launch_dependents();
-  const int KB = K / kSfBlock;
-  const int n_rt = sf_row_atoms(cap);
-  const int n_kt = sf_k_atoms(K);
+  const int KB = a.K / kSfBlock;
+  const int n_rt = sf_row_atoms(a.cap);
+  const int n_kt = sf_k_atoms(a.K);
+  const bool wide = (reinterpret_cast<uintptr_t>(a.x) & 31) == 0;
   const int lane = threadIdx.x & 31;
-  const unsigned slots = (unsigned)E * (unsigned)cap;
-  const unsigned warp0 = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  LiveRows rows;
+  rows.make(a.counts, a.E, a.cap, s_prefix);
   const unsigned nwarps = gridDim.x * kWarpsPerBlock;
-  for (unsigned slot = warp0; slot < slots; slot += nwarps) {
-    const int e = (int)(slot / (unsigned)cap);
-    const int r = (int)(slot - (unsigned)e * (unsigned)cap);
-    if (r >= min(counts[e], cap)) {
-      // jump to the next expert's first slot that this warp owns
-      const unsigned next = (unsigned)(e + 1) * (unsigned)cap;
-      const unsigned skip = (next - slot + nwarps - 1) / nwarps;
-      slot += (skip - 1) * nwarps;
-      continue;
-    }
-    const float gs = gscale_per_expert ? gscale[e] : gscale[0];
-    const bool weighted = topk_w != nullptr;
-    const float w = weighted ? __bfloat162float(__float2bfloat16_rn(topk_w[src_route[slot]])) : 1.f;
-    quantize_routed_row(reinterpret_cast<const uint4*>(a1 + (long long)src_tok[slot] * K),
-                        reinterpret_cast<uint4*>(b_act + (long long)slot * (K / 2)), sfb + sf_offset(e, r, 0, n_rt, n_kt),
-                        KB, gs, weighted, w, lane);
+  // With fewer rows than warps a row is cut into pieces of 32 K-blocks or more: a decode step then takes as long as one
+  // piece.  (Consecutive warps take consecutive rows of one piece; the scale words of 32 rows share lines.)
+  unsigned pieces = 1;
+  int piece_blocks = KB;
+  if (rows.total > 0 && 2u * rows.total <= nwarps && KB > 32) {
+    pieces = min(nwarps / rows.total, (unsigned)(KB + 31) / 32u);
+    piece_blocks = (int)(((unsigned)KB + pieces - 1) / pieces + 31) / 32 * 32;
+    pieces = (unsigned)(KB + piece_blocks - 1) / (unsigned)piece_blocks;
   }
+  const unsigned units = rows.total * pieces;
+  const long long row_bytes = (kSrc == kGated ? 4LL : 2LL) * a.K;
+  for (unsigned u = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); u < units; u += nwarps) {
+    const unsigned piece = pieces > 1 ? u / rows.total : 0u;
+    int e, r;
+    if (!rows.find(u - piece * rows.total, e, r)) continue;
+    const long long slot = (long long)e * a.cap + r;
+    const int lo = (int)piece * piece_blocks, hi = min(KB, lo + piece_blocks);
+    const float gs = a.gscale_per_expert ? a.gscale[e] : a.gscale[0];
+    const bool weighted = kSrc == kGather && a.topk_w != nullptr;
+    float w = 1.f;
+    long long src_row = slot;
+    if constexpr (kSrc == kGather) {
+      src_row = a.src_tok[slot];
+      if (weighted) w = __bfloat162float(__float2bfloat16_rn(a.topk_w[a.src_route[slot]]));
+    }
+    const uint8_t* src = reinterpret_cast<const uint8_t*>(a.x) + src_row * row_bytes;
+    uint4* dst = reinterpret_cast<uint4*>(a.b_act + slot * (a.K / 2));
+    uint8_t* sf_row = a.sfb + sf_offset(e, r, 0, n_rt, n_kt);
+    for (int kb0 = lo; kb0 < hi; kb0 += 32) {
+      BlockRegs b;
+      const int kb = kb0 + lane;
+      if (kb < KB) {
+        if constexpr (kSrc == kGated) {
+          const uint8_t* gate = src + (a.interleaved ? 128LL : 64LL) * kb;
+          const uint8_t* up = a.interleaved ? gate + 64 : gate + 64LL * KB;
+          BlockRegs g, up_b;
+          load_block(gate, wide, g);
+          load_block(up, wide, up_b);
+          gated_act16(g.lo, up_b.lo, a.act, b.lo);
+          gated_act16(g.hi, up_b.hi, a.act, b.hi);
+        } else {
+          load_block(src + 64LL * kb, wide, b);
+          if (weighted) block_weight(b, w);
+        }
+      }
+      finish_blocks(b, kb0, KB, gs, dst, sf_row, lane);
+    }
+  }
+  benign_fill_dead(a.counts, a.E, a.cap, n_rt, n_kt, a.sfb);
 }
 
-// scatter_fp4_planned / scatter_fp4_wire: already quantized rows into the batched operands, one warp per row slot.
+// n 16-byte words by one warp, eight of them per lane in flight.
+__device__ __forceinline__ void warp_copy(const uint4* __restrict__ src, uint4* __restrict__ dst, int n, int lane) {
+  for (int v0 = 0; v0 < n; v0 += 256) {
+    uint4 x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (v0 + i * 32 + lane < n) x[i] = __ldg(src + v0 + i * 32 + lane);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (v0 + i * 32 + lane < n) dst[v0 + i * 32 + lane] = x[i];
+  }
+}
+constexpr int kCopyBlocks = 3;      // blocks per SM of the kernels that copy rows (80 registers)
+
+// scatter_fp4_planned / scatter_fp4_wire: already quantized rows into the batched operands, one warp per live row.
 // Codes are copied 16 bytes per lane; the row's scales go from natural order into the swizzled layout four
-// K-blocks (one aligned word of both layouts) at a time.  Slots at or past counts[e] are skipped; their scales
-// keep the benign fill laid down before the launch.
+// K-blocks (one aligned word of both layouts) at a time.  Slots at or past counts[e] get the benign fill in their scales.
+// Bound: HBM (65536 rows of 7168: 250 MB in and out in 104 us; a plain fill of 256 MB takes 74).
 __global__ void __launch_bounds__(kThreads)
 scatter_fp4_rows_kernel(const uint8_t* __restrict__ q, long long q_pitch, const uint8_t* __restrict__ q_sf,
                         long long sf_pitch, const int* __restrict__ src_tok, const int* __restrict__ counts, int K, int E,
                         int cap, uint8_t* __restrict__ b_act, uint8_t* __restrict__ sfb) {
+  extern __shared__ int s_prefix[];
   pdl_wait();
   pdl_launch_dependents();
   const int KB = K / kSfBlock;
   const int n_rt = sf_row_atoms(cap);
   const int n_kt = sf_k_atoms(K);
   const int lane = threadIdx.x & 31;
-  const unsigned slots = (unsigned)E * (unsigned)cap;
-  const unsigned warp0 = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  LiveRows rows;
+  rows.make(counts, E, cap, s_prefix);
   const unsigned nwarps = gridDim.x * kWarpsPerBlock;
   const bool words = (KB % 4) == 0 && (sf_pitch % 4) == 0 && (reinterpret_cast<uintptr_t>(q_sf) % 4) == 0;
-  for (unsigned slot = warp0; slot < slots; slot += nwarps) {
-    const int e = (int)(slot / (unsigned)cap);
-    const int r = (int)(slot - (unsigned)e * (unsigned)cap);
-    if (r >= min(counts[e], cap)) {
-      const unsigned next = (unsigned)(e + 1) * (unsigned)cap;       // on to the next expert's first slot of this warp
-      slot += ((next - slot + nwarps - 1) / nwarps - 1) * nwarps;
-      continue;
-    }
+  for (unsigned j = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); j < rows.total; j += nwarps) {
+    int e, r;
+    if (!rows.find(j, e, r)) continue;
+    const long long slot = (long long)e * cap + r;
     const long long t = src_tok[slot];
-    const uint4* src = reinterpret_cast<const uint4*>(q + t * q_pitch);
-    uint4* dst = reinterpret_cast<uint4*>(b_act + (long long)slot * (K / 2));
-    for (int v = lane; v < K / 32; v += 32) dst[v] = __ldg(src + v);
     const uint8_t* sf_src = q_sf + t * sf_pitch;
     uint8_t* sf_row = sfb + sf_offset(e, r, 0, n_rt, n_kt);        // K-block kb of this row: + (kb >> 2) * 512 + (kb & 3)
     if (words) {
       for (int w = lane; w < KB / 4; w += 32)
         *reinterpret_cast<uint32_t*>(sf_row + w * 512) = __ldg(reinterpret_cast<const uint32_t*>(sf_src) + w);
     } else {
-      for (int kb = lane; kb < KB; kb += 32) sf_row[(kb >> 2) * 512 + (kb & 3)] = __ldg(sf_src + kb);
+      for (int kb = lane; kb < n_kt * 4; kb += 32)      // (blocks past K keep the benign byte in the layout's slop)
+        sf_row[(kb >> 2) * 512 + (kb & 3)] = kb < KB ? __ldg(sf_src + kb) : (uint8_t)kBenignSf;
     }
+    warp_copy(reinterpret_cast<const uint4*>(q + t * q_pitch), reinterpret_cast<uint4*>(b_act + slot * (K / 2)), K / 32, lane);
   }
+  benign_fill_dead(counts, E, cap, n_rt, n_kt, sfb);
 }
 
 // quant_rows: token-order rows -> row-major codes and natural-order scales, one shared global scale.
@@ -294,8 +370,9 @@ quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
   const unsigned warp0 = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const unsigned nwarps = gridDim.x * kWarpsPerBlock;
   const bool sf_words = (KB % 4) == 0;     // rows of scales are then 4-byte aligned
+  const bool wide = (reinterpret_cast<uintptr_t>(x) & 31) == 0;
   for (unsigned t = warp0; t < T; t += nwarps) {
-    const uint4* src = reinterpret_cast<const uint4*>(x + (long long)t * K);
+    const uint8_t* src = reinterpret_cast<const uint8_t*>(x + (long long)t * K);
     uint4* dst = reinterpret_cast<uint4*>(q + (long long)t * (K / 2));
     uint8_t* sf_row = q_sf + (long long)t * KB;
     for (int kb0 = 0; kb0 < KB; kb0 += 32) {
@@ -303,7 +380,7 @@ quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
       uint32_t sf_byte = 0;
       if (kb < KB) {
         BlockRegs b;
-        load_block(src + kb * 4, b);
+        load_block(src + 64LL * kb, wide, b);
         float inv;
         block_scale(block_amax(b), gs, sf_byte, inv);
         dst[kb] = block_codes(b, inv);
@@ -346,45 +423,48 @@ gated_act_kernel(const __nv_bfloat16* __restrict__ x2, long long rows, int N, in
 // treats like any routing that is not for one of its experts.
 __host__ __device__ inline long long wire_row_bytes(int K) { return (long long)round_up_i(K / 2 + K / kSfBlock, 16) + 16; }
 
+// One warp per slot, all of a row's words in flight at once.  Bound: writes to HBM (65536 rows of 3840 bytes: 75 us, as a
+// plain fill of as many bytes; with a block of 128 threads per slot and its three dependent loads 85).
 template <class IdT>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kThreads)
 pack_wire_rows_kernel(const uint8_t* __restrict__ q, const uint8_t* __restrict__ q_sf, const IdT* __restrict__ ids,
                       const int* __restrict__ slot_tok, const int* __restrict__ slot_route,
-                      const int* __restrict__ slab_counts, int slab, int experts_per_rank, int K,
+                      const int* __restrict__ slab_counts, unsigned slots, int slab, int experts_per_rank, int K,
                       uint8_t* __restrict__ wire, const RowParts parts) {
   pdl_wait();
   pdl_launch_dependents();
-  const long long slot = blockIdx.x;
-  const int w = (int)(slot / slab);
-  const int s = (int)(slot - (long long)w * slab);
   const long long row_bytes = wire_row_bytes(K);
-  // (with parts: slab w goes to buffer w, which may be the receiving rank's own memory)
-  uint8_t* row = parts.n ? static_cast<uint8_t*>(parts.base[w]) + s * row_bytes : wire + slot * row_bytes;
-  int* id_out = reinterpret_cast<int*>(row + row_bytes - 16);
-  if (s >= min(slab_counts[w], slab)) {
-    if (threadIdx.x == 0) *id_out = -1;
-    return;
-  }
-  const long long t = slot_tok[slot];
-  const int code_vecs = K / 32;                       // 16-byte words of codes
-  const uint4* src = reinterpret_cast<const uint4*>(q + t * (K / 2));
-  uint4* dst = reinterpret_cast<uint4*>(row);
-  for (int v = threadIdx.x; v < code_vecs; v += 128) dst[v] = __ldg(src + v);
   const int KB = K / kSfBlock;
-  const uint8_t* sf_src = q_sf + t * KB;
-  uint8_t* sf_dst = row + K / 2;
-  if (KB % 16 == 0) {
-    for (int v = threadIdx.x; v < KB / 16; v += 128)
-      reinterpret_cast<uint4*>(sf_dst)[v] = __ldg(reinterpret_cast<const uint4*>(sf_src) + v);
-  } else {
-    for (int b = threadIdx.x; b < KB; b += 128) sf_dst[b] = __ldg(sf_src + b);
+  const int lane = threadIdx.x & 31;
+  const unsigned nwarps = gridDim.x * kWarpsPerBlock;
+  for (unsigned slot = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); slot < slots; slot += nwarps) {
+    const int w = (int)(slot / (unsigned)slab);
+    const int s = (int)(slot - (unsigned)w * (unsigned)slab);
+    // (with parts: slab w goes to buffer w, which may be the receiving rank's own memory)
+    uint8_t* row = parts.n ? static_cast<uint8_t*>(parts.base[w]) + s * row_bytes : wire + slot * row_bytes;
+    int* id_out = reinterpret_cast<int*>(row + row_bytes - 16);
+    if (s >= min(slab_counts[w], slab)) {
+      if (lane == 0) *id_out = -1;
+      continue;
+    }
+    const long long t = slot_tok[slot];
+    const int route = slot_route[slot];
+    const uint8_t* sf_src = q_sf + t * KB;
+    uint8_t* sf_dst = row + K / 2;
+    if (KB % 16 == 0) {
+      for (int v = lane; v < KB / 16; v += 32)
+        reinterpret_cast<uint4*>(sf_dst)[v] = __ldg(reinterpret_cast<const uint4*>(sf_src) + v);
+    } else {
+      for (int b = lane; b < KB; b += 32) sf_dst[b] = __ldg(sf_src + b);
+    }
+    warp_copy(reinterpret_cast<const uint4*>(q + t * (K / 2)), reinterpret_cast<uint4*>(row), K / 32, lane);
+    if (lane == 0) *id_out = (int)((long long)ids[route] - (long long)w * experts_per_rank);
   }
-  if (threadIdx.x == 0) *id_out = (int)((long long)ids[slot_route[slot]] - (long long)w * experts_per_rank);
 }
 
-int grid_for(long long warp_items, int sm_count) {
+int grid_for(long long warp_items, int sm_count, int per_sm = 8) {      // 8 x 256 threads fill an SM
   long long blocks = (warp_items + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  long long cap = (long long)(sm_count > 0 ? sm_count : 148) * 8;   // 8 x 256 threads fill an SM
+  long long cap = (long long)(sm_count > 0 ? sm_count : 148) * per_sm;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
   return (int)blocks;
@@ -397,6 +477,16 @@ int check_common(const void* x, const float* gscale, const int32_t* counts, int 
   PNV_REQUIRE(K > 0 && K % kSfBlock == 0, "%s must be a multiple of %d, got %d", kname, kSfBlock, K);
   PNV_REQUIRE(sf_numel(rows, K, E) / 16 < (1LL << 31) - (1LL << 24), "the scale layout has too many lines for one launch");
   PNV_REQUIRE(sf_numel(rows, K, E) / 16 < (1LL << 40), "scale buffer too large");
+  return PNV_OK;
+}
+
+// One launch of the shared kernel: at most a wave of warps, one per 32 K-blocks of a row of the capacity.
+template <int kSrc>
+int launch_batched(const RowsArgs& a, int sm_count, cudaStream_t s) {
+  PNV_REQUIRE((long long)a.E * a.cap < (1LL << 31), "E * cap must fit int32");
+  const long long units = (long long)a.E * a.cap * ceil_div_i(a.K / kSfBlock, 32);
+  PNV_CUDA(launch_pdl(quant_batched_kernel<kSrc>, dim3(grid_for(units, sm_count, kBatchedBlocks)), dim3(kThreads),
+                      live_rows_smem(a.E), s, pdl_enabled(), a));
   return PNV_OK;
 }
 
@@ -424,12 +514,9 @@ extern "C" int pnv_quant_act(const void* x, const float* gscale, int gscale_per_
                              const int32_t* counts, int experts, int max_n, int k, uint8_t* b_act,
                              uint8_t* sfb, int sm_count, pnv_stream_t stream) {
   if (int rc = check_common(x, gscale, counts, experts, max_n, k, b_act, sfb, "K")) return rc;
-  long long lines = sf_numel(max_n, k, experts) / 16;
-  GatedAct act{};
-  PNV_CUDA(launch_pdl(quant_lines_kernel<kPlain>, dim3(grid_for(lines, sm_count)), dim3(kThreads), 0,
-                      (cudaStream_t)stream, pdl_enabled(), (const __nv_bfloat16*)x, gscale,
-                      gscale_per_expert, counts, experts, max_n, k, 0, act, b_act, sfb));
-  return PNV_OK;
+  RowsArgs a{(const __nv_bfloat16*)x, nullptr, nullptr, nullptr, gscale, (const int*)counts, b_act, sfb, GatedAct{},
+             gscale_per_expert, experts, max_n, k, 0};
+  return launch_batched<kPlain>(a, sm_count, (cudaStream_t)stream);
 }
 
 extern "C" int pnv_silu_mul_quant_act(const void* x2, const float* gscale, int gscale_per_expert,
@@ -441,12 +528,9 @@ extern "C" int pnv_silu_mul_quant_act(const void* x2, const float* gscale, int g
   if (int rc = make_gated_act(act_kind, beta, linear_beta, act)) return rc;
   if (int rc = check_common(x2, gscale, counts, experts, max_n, n, b_act, sfb, "intermediate width N"))
     return rc;
-  long long lines = sf_numel(max_n, n, experts) / 16;
-  PNV_CUDA(launch_pdl(quant_lines_kernel<kGated>, dim3(grid_for(lines, sm_count)), dim3(kThreads), 0,
-                      (cudaStream_t)stream, pdl_enabled(), (const __nv_bfloat16*)x2, gscale,
-                      gscale_per_expert, counts, experts, max_n, n, interleaved ? 1 : 0, act,
-                      b_act, sfb));
-  return PNV_OK;
+  RowsArgs a{(const __nv_bfloat16*)x2, nullptr, nullptr, nullptr, gscale, (const int*)counts, b_act, sfb, act,
+             gscale_per_expert, experts, max_n, n, interleaved ? 1 : 0};
+  return launch_batched<kGated>(a, sm_count, (cudaStream_t)stream);
 }
 
 extern "C" int pnv_scatter_quant_act(const void* a1, const int64_t* flat_tok,
@@ -495,14 +579,9 @@ extern "C" int pnv_scatter_quant_act_planned(const void* a1, const int32_t* src_
   PNV_REQUIRE(cap > 0, "cap must be positive");
   PNV_REQUIRE(src_tok && src_route, "null pointer argument");
   if (int rc = check_common(a1, gscale, counts, experts, cap, k, b_act, sfb, "K")) return rc;
-  PNV_REQUIRE((long long)experts * cap < (1LL << 31), "E * cap must fit int32");
-  cudaStream_t s = (cudaStream_t)stream;
-  // benign fill first, then one warp per live row writes its scales over it
-  PNV_CUDA(cudaMemsetAsync(sfb, kBenignSf, (size_t)sf_numel(cap, k, experts), s));
-  PNV_CUDA(launch_pdl(scatter_planned_rows_kernel, dim3(grid_for((long long)experts * cap, sm_count)), dim3(kThreads), 0, s,
-                      false, (const __nv_bfloat16*)a1, (const int*)src_tok, (const int*)src_route, topk_weights, gscale,
-                      gscale_per_expert, (const int*)counts, k, experts, cap, b_act, sfb));
-  return PNV_OK;
+  RowsArgs a{(const __nv_bfloat16*)a1, (const int*)src_tok, (const int*)src_route, topk_weights, gscale, (const int*)counts,
+             b_act, sfb, GatedAct{}, gscale_per_expert, experts, cap, k, 0};
+  return launch_batched<kGather>(a, sm_count, (cudaStream_t)stream);
 }
 
 extern "C" int pnv_quant_rows(const void* x, const float* gscale, int64_t tokens, int k, uint8_t* q, uint8_t* q_sf,
@@ -526,11 +605,9 @@ int scatter_fp4_rows(const uint8_t* q, long long q_pitch, const uint8_t* q_sf, l
   PNV_REQUIRE((long long)experts * cap < (1LL << 31), "E * cap must fit int32");
   PNV_REQUIRE((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(b_act) | (uintptr_t)q_pitch) % 16 == 0,
               "code rows must be 16-byte aligned");
-  // benign fill first, then one warp per live row writes its scales over it
-  PNV_CUDA(cudaMemsetAsync(sfb, kBenignSf, (size_t)sf_numel(cap, k, experts), s));
-  PNV_CUDA(launch_pdl(scatter_fp4_rows_kernel, dim3(grid_for((long long)experts * cap, sm_count)), dim3(kThreads), 0, s,
-                      false, q, q_pitch, q_sf, sf_pitch, (const int*)src_tok, (const int*)counts, k, experts, cap, b_act,
-                      sfb));
+  PNV_CUDA(launch_pdl(scatter_fp4_rows_kernel, dim3(grid_for((long long)experts * cap, sm_count, kCopyBlocks)), dim3(kThreads),
+                      live_rows_smem(experts), s, pdl_enabled(), q, q_pitch, q_sf, sf_pitch, (const int*)src_tok,
+                      (const int*)counts, k, experts, cap, b_act, sfb));
   return PNV_OK;
 }
 }  // namespace
@@ -569,14 +646,15 @@ int pack_wire_rows_common(const uint8_t* q, const uint8_t* q_sf, const void* top
                   ((k / kSfBlock) % 16 != 0 || reinterpret_cast<uintptr_t>(q_sf) % 16 == 0),
               "pack_wire_rows buffers must be 16-byte aligned");
   cudaStream_t s = (cudaStream_t)stream;
-  const dim3 grid((unsigned)(ranks * slab)), block(128);
+  const unsigned slots = (unsigned)(ranks * slab);
+  const dim3 grid((unsigned)grid_for(slots, 0, kCopyBlocks)), block(kThreads);
   if (ids_are_int64)
     PNV_CUDA(launch_pdl(pack_wire_rows_kernel<long long>, grid, block, 0, s, pdl_enabled(), q, q_sf,
                         (const long long*)topk_ids, (const int*)slot_tok, (const int*)slot_route,
-                        (const int*)slab_counts, slab, experts_per_rank, k, wire, parts));
+                        (const int*)slab_counts, slots, slab, experts_per_rank, k, wire, parts));
   else
     PNV_CUDA(launch_pdl(pack_wire_rows_kernel<int>, grid, block, 0, s, pdl_enabled(), q, q_sf, (const int*)topk_ids,
-                        (const int*)slot_tok, (const int*)slot_route, (const int*)slab_counts, slab,
+                        (const int*)slot_tok, (const int*)slot_route, (const int*)slab_counts, slots, slab,
                         experts_per_rank, k, wire, parts));
   return PNV_OK;
 }
