@@ -159,6 +159,7 @@ __device__ __forceinline__ __nv_bfloat16* mapped_row(const Params& p, long long 
 // active experts (counts > 0) in shared memory no role walks over the idle ones.  One token on 8 of 128 experts, 2048 x
 // 1536 and 768 x 2048 weights: 16 and 17 us per GEMM with that walk and with K always split, 6.5 and 5.4 us now.
 constexpr int kSplitSaves = 6;
+static_assert(PNV_SPLIT_MIN_K == kSplitSaves * 512 + 1, "the smallest K of kSplitSaves + 1 stages");
 struct UnitWalk {
   const unsigned short* active;      // the active experts in order
   unsigned n_tiles, n_mt;
@@ -1053,7 +1054,7 @@ int group_mm_common(void* out, const int32_t* row_map, const RowParts* out_parts
   p.k_stages = ceil_div_i(k, stage_k);
   // the split schedule counts K stages in 32 bits
   const bool split_fits = (long long)experts * p.n_mt * p.k_stages < (1LL << 30);
-  if (narrow && workspace != nullptr && p.k_stages > 1 && split_fits) {
+  if (narrow && workspace != nullptr && k >= PNV_SPLIT_MIN_K && split_fits) {
     const int64_t need = pnv_group_mm_workspace_bytes(experts, features, max_n, sm_count);
     PNV_REQUIRE(workspace_bytes >= need, "group_mm: the split-K workspace holds %lld bytes, %lld are needed",
                 (long long)workspace_bytes, (long long)need);

@@ -475,11 +475,13 @@ struct Workspace {
 };
 constexpr size_t kMaxWorkspaces = 32;
 
-Tensor split_workspace(const Tensor& t, cudaStream_t stream, int64_t experts, int64_t features, int64_t max_n, int64_t* bytes) {
+Tensor split_workspace(const Tensor& t, cudaStream_t stream, int64_t experts, int64_t features, int64_t k, int64_t max_n, int64_t* bytes) {
   static std::mutex mu;
   static std::list<Workspace>* pool = new std::list<Workspace>;      // never destroyed: tensors must not outlive CUDA at exit
   const int sms = sm_count(t);
-  *bytes = pnv_group_mm_workspace_bytes((int)experts, (int)features, (int)max_n, sms);
+  // (a K too short to be split needs none: in a captured decode step the clearing of its counters was a node of its own
+  // between two GEMMs and kept the second from starting early: 101.0 -> 99.3 us for 128 tokens on 32 experts)
+  *bytes = k < PNV_SPLIT_MIN_K ? 0 : pnv_group_mm_workspace_bytes((int)experts, (int)features, (int)max_n, sms);
   if (*bytes == 0) return Tensor();
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
@@ -553,7 +555,7 @@ void group_mm_impl(const Tensor* out, const at::TensorList* out_parts, const Ten
   const c10::cuda::CUDAGuard guard(b_act.device());
   const cudaStream_t stream = current_stream(b_act);
   int64_t ws_bytes = 0;
-  const Tensor ws = split_workspace(b_act, stream, E, M, max_n, &ws_bytes);
+  const Tensor ws = split_workspace(b_act, stream, E, M, K, max_n, &ws_bytes);
   void* ws_ptr = ws.defined() ? ws.data_ptr() : nullptr;
   const int e = (int)E, m = (int)M, k = (int)K, n = (int)max_n, cfg = (int)config_id, cm = (int)cluster_m, cn = (int)cluster_n;
   const int sms = sm_count(b_act);
@@ -613,7 +615,7 @@ std::tuple<Tensor, Tensor> group_mm_swiglu_quant(const Tensor& a_comp, const Ten
   const c10::cuda::CUDAGuard guard(b_act.device());
   const cudaStream_t stream = current_stream(b_act);
   int64_t ws_bytes = 0;
-  const Tensor ws = split_workspace(b_act, stream, E, M, max_n, &ws_bytes);
+  const Tensor ws = split_workspace(b_act, stream, E, M, K, max_n, &ws_bytes);
   check_rc(pnv_group_mm_swiglu_quant(b_out.mutable_data_ptr<uint8_t>(), sfb_out.mutable_data_ptr<uint8_t>(), u8(a_comp), u8(e_meta),
                                      u8(sfa), u8(b_act), u8(sfb), f32(alphas), i32(counts), f32(gscale), gscale.numel() == E, (int)E,
                                      (int)M, (int)K, (int)max_n, (int)config_id, (int)cluster_m, (int)cluster_n, kind, (float)beta,
