@@ -675,22 +675,28 @@ TORCH_LIBRARY(paired_nvfp4, m) {
   m.def("gated_act(Tensor x2, bool interleaved=False, str activation=\"silu\", float beta=1.0, float linear_beta=-1.0) -> Tensor");
 }
 
-#define PNV_OPS(X)                                                                                                     \
+// The operators whose results are whole numbers (codes, scales, plans) or that only write into their arguments ...
+#define PNV_OPS_WITHOUT_FLOAT_RESULTS(X)                                                                               \
   X(compress) X(quant_act) X(silu_mul_quant_act) X(scatter_quant_act) X(dispatch_plan) X(scatter_quant_act_planned)     \
-  X(quant_rows) X(scatter_fp4_planned) X(moe_finalize) X(gather_rows) X(pack_wire_rows) X(scatter_fp4_wire) X(group_mm) \
-  X(group_mm_rows) X(zero_rows) X(group_mm_rows_parts) X(zero_rows_parts) X(pack_wire_rows_parts) X(gated_act)          \
+  X(quant_rows) X(scatter_fp4_planned) X(moe_finalize) X(pack_wire_rows) X(scatter_fp4_wire) X(group_mm)                \
+  X(group_mm_rows) X(zero_rows) X(group_mm_rows_parts) X(zero_rows_parts) X(pack_wire_rows_parts)                       \
   X(group_mm_swiglu_quant)
+// ... and those that return floating-point tensors
+#define PNV_OPS_WITH_FLOAT_RESULTS(X) X(gather_rows) X(gated_act)
 
 TORCH_LIBRARY_IMPL(paired_nvfp4, CUDA, m) {
 #define PNV_IMPL(name) m.impl(#name, TORCH_FN(name));
-  PNV_OPS(PNV_IMPL)
+  PNV_OPS_WITHOUT_FLOAT_RESULTS(PNV_IMPL)
+  PNV_OPS_WITH_FLOAT_RESULTS(PNV_IMPL)
 #undef PNV_IMPL
 }
 
-// There is no backward for these ops: skip the (boxed) autograd fallback.
+// There is no backward for these ops.  torch's autograd fallback says so by a node on every floating-point result of an
+// input that requires grad, which warns in backward; it never touches integer results or written arguments, so the ops
+// without floating-point results skip it (it is boxed: a microsecond or two a call).
 TORCH_LIBRARY_IMPL(paired_nvfp4, AutogradCUDA, m) {
 #define PNV_FALLTHROUGH(name) m.impl(#name, torch::CppFunction::makeFallthrough());
-  PNV_OPS(PNV_FALLTHROUGH)
+  PNV_OPS_WITHOUT_FLOAT_RESULTS(PNV_FALLTHROUGH)
 #undef PNV_FALLTHROUGH
 }
 
