@@ -460,20 +460,27 @@ Tensor gated_act(const Tensor& x2, bool interleaved, c10::string_view activation
 // ---- grouped GEMM --------------------------------------------------------------------------------------
 
 // Split-K workspaces (the reference allocates its workspace inside the op as well, csrc/group_mm.cuh:163-165).  One is
-// kept per (device, stream, size), and per capture while the stream is being captured, so a graph never shares a buffer
-// with work outside it; the counters are zeroed when a workspace is made and every launch leaves them zero.  Launches
-// with another number of counters get a workspace of their own: the partial sums follow the counters, so in a shared
-// one a launch would leave its sums where the other's counters are.
+// kept per (device, stream, size); the counters are zeroed when a workspace is made and every launch leaves them zero.
+// Launches with another number of counters get a workspace of their own: the partial sums follow the counters, so in a
+// shared one a launch would leave its sums where the other's counters are.
 // The list is short and least recently used entries go back to the caching allocator; a workspace is allocated with its
 // stream current, so what the allocator does with a returned one is ordered after the launches that used it.
+// While the stream is being captured nothing is kept: the call makes a workspace in the capture's memory pool, zeroes its
+// counters inside the graph and gives it back when it returns, like any temporary of the captured program, so a graph never
+// shares a buffer with work outside it and holds no memory that outlives it.
 struct Workspace {
   int device;
   cudaStream_t stream;
-  unsigned long long capture;
   int64_t counters, bytes;
   Tensor buf;
 };
 constexpr size_t kMaxWorkspaces = 32;
+
+Tensor new_workspace(const Tensor& t, cudaStream_t stream, int64_t counters, int64_t bytes) {
+  Tensor buf = empty_on(t, {bytes}, at::kByte);
+  TORCH_CHECK(cudaMemsetAsync(buf.data_ptr(), 0, (size_t)counters, stream) == cudaSuccess, "cudaMemsetAsync failed");
+  return buf;
+}
 
 Tensor split_workspace(const Tensor& t, cudaStream_t stream, int64_t experts, int64_t features, int64_t k, int64_t max_n, int64_t* bytes) {
   static std::mutex mu;
@@ -483,23 +490,21 @@ Tensor split_workspace(const Tensor& t, cudaStream_t stream, int64_t experts, in
   // between two GEMMs and kept the second from starting early: 101.0 -> 99.3 us for 128 tokens on 32 experts)
   *bytes = k < PNV_SPLIT_MIN_K ? 0 : pnv_group_mm_workspace_bytes((int)experts, (int)features, (int)max_n, sms);
   if (*bytes == 0) return Tensor();
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  unsigned long long id = 0;
-  TORCH_CHECK(cudaStreamGetCaptureInfo(stream, &status, &id) == cudaSuccess, "cudaStreamGetCaptureInfo failed");
-  if (status == cudaStreamCaptureStatusNone) id = 0;
-  const int dev = t.get_device();
   // the counters, one per (expert, 128 features), come first and are the only part that has to start at zero
   const int64_t counters = std::min<int64_t>(*bytes, ceil_div(experts * ceil_div(features, 128) * 4, 256) * 256);
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  TORCH_CHECK(cudaStreamIsCapturing(stream, &status) == cudaSuccess, "cudaStreamIsCapturing failed");
+  if (status != cudaStreamCaptureStatusNone) return new_workspace(t, stream, counters, *bytes);
+  const int dev = t.get_device();
   std::lock_guard<std::mutex> lock(mu);
   for (auto it = pool->begin(); it != pool->end(); ++it) {
-    if (it->device == dev && it->stream == stream && it->capture == id && it->counters == counters && it->bytes == *bytes) {
+    if (it->device == dev && it->stream == stream && it->counters == counters && it->bytes == *bytes) {
       pool->splice(pool->begin(), *pool, it);
       return pool->front().buf;
     }
   }
-  Tensor buf = empty_on(t, {*bytes}, at::kByte);
-  TORCH_CHECK(cudaMemsetAsync(buf.data_ptr(), 0, (size_t)counters, stream) == cudaSuccess, "cudaMemsetAsync failed");
-  pool->push_front(Workspace{dev, stream, id, counters, *bytes, buf});
+  Tensor buf = new_workspace(t, stream, counters, *bytes);
+  pool->push_front(Workspace{dev, stream, counters, *bytes, buf});
   if (pool->size() > kMaxWorkspaces) pool->pop_back();
   return buf;
 }
