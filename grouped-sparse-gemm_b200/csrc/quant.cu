@@ -73,7 +73,8 @@ __device__ __forceinline__ void block_weight(BlockRegs& b, float w) {
 enum RowSource : int { kPlain = 0, kGated = 1, kGather = 2 };
 
 // 32 K-blocks from kb0 on, one per lane in b, are scaled, rounded and stored; a row's four scales of one 128-K group are one
-// aligned word of the swizzled layout.  KB: the blocks of the whole row.
+// aligned word of the swizzled layout.  KB: the blocks of the whole row.  kLoose: the codes are 8-byte aligned only.
+template <bool kLoose = false>
 __device__ __forceinline__ void finish_blocks(const BlockRegs& b, int kb0, int KB, float gs, uint4* __restrict__ dst,
                                               uint8_t* __restrict__ sf_row, int lane) {
   const int kb = kb0 + lane;
@@ -81,7 +82,14 @@ __device__ __forceinline__ void finish_blocks(const BlockRegs& b, int kb0, int K
   if (kb < KB) {
     float inv;
     block_scale(block_amax(b), gs, sf_byte, inv);
-    dst[kb] = block_codes(b, inv);
+    const uint4 codes = block_codes(b, inv);
+    if constexpr (!kLoose) {
+      dst[kb] = codes;
+    } else {
+      uint2* half = reinterpret_cast<uint2*>(dst + kb);
+      half[0] = make_uint2(codes.x, codes.y);
+      half[1] = make_uint2(codes.z, codes.w);
+    }
   }
   const uint32_t word = gather_sf_word(sf_byte);
   if ((lane & 3) == 0 && kb < KB) *reinterpret_cast<uint32_t*>(sf_row + (kb >> 2) * 512) = word;
@@ -124,23 +132,34 @@ scatter_quant_kernel(const __nv_bfloat16* __restrict__ a1, const long long* __re
 // Every byte of a scale buffer that no live row (r < counts[e]) writes becomes 0x38: whole 16-byte lines behind which
 // no row is live, single words of the others.  (K-block slop of a live row is part of the words that row writes.)  The
 // kernels that place rows do this themselves, each thread a share of the lines: as a memset in front of them it was a
-// launch of its own and kept them from starting while their predecessor drains.
+// launch of its own and kept them from starting while their predecessor drains.  (kLoose: the buffer may be less than
+// 16-byte aligned, and is then filled word by word, or byte by byte.)
+template <bool kLoose>
 __device__ __forceinline__ void benign_fill_dead(const int* __restrict__ counts, int E, int cap, int n_rt, int n_kt,
                                                  uint8_t* __restrict__ sfb) {
   const uint32_t w4 = kBenignSf * 0x01010101u;
   const unsigned lines = (unsigned)E * n_rt * n_kt * 32u;
+  const bool sfb16 = !kLoose || (reinterpret_cast<uintptr_t>(sfb) & 15) == 0;
+  const bool sfb4 = !kLoose || (reinterpret_cast<uintptr_t>(sfb) & 3) == 0;
   for (unsigned c = blockIdx.x * kThreads + threadIdx.x; c < lines; c += gridDim.x * kThreads) {
     const unsigned a_kt = (c >> 5) / (unsigned)n_kt;
     const unsigned e = a_kt / (unsigned)n_rt;
     const int r0 = (int)(a_kt - e * (unsigned)n_rt) * 128 + (int)(c & 31);
     const int cnt = min(counts[e], cap);
     uint8_t* line = sfb + (long long)c * 16;
-    if (r0 >= cnt) {
+    if (r0 >= cnt && sfb16) {
       *reinterpret_cast<uint4*>(line) = make_uint4(w4, w4, w4, w4);
     } else {
 #pragma unroll
-      for (int g = 1; g < 4; ++g)
-        if (r0 + 32 * g >= cnt) *reinterpret_cast<uint32_t*>(line + 4 * g) = w4;
+      for (int g = 0; g < 4; ++g)
+        if (r0 + 32 * g >= cnt) {
+          if (sfb4) {
+            *reinterpret_cast<uint32_t*>(line + 4 * g) = w4;
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) line[4 * g + i] = (uint8_t)kBenignSf;
+          }
+        }
     }
   }
 }
@@ -240,7 +259,9 @@ struct RowsArgs {
 // next step's loads ahead of the arithmetic are 15 % slower.  The grid is one wave of them.
 constexpr int kBatchedBlocks = 4;
 
-template <int kSrc>
+// kLoose: codes or scales that are less than 16-byte aligned (pieces of a caller's larger buffer).  A form of its own,
+// because with the tests at run time the activation's form spilled and ran 1 % longer.
+template <int kSrc, bool kLoose>
 __global__ void __launch_bounds__(kThreads, kBatchedBlocks)
 quant_batched_kernel(const RowsArgs a) {
   extern __shared__ int s_prefix[];
@@ -299,10 +320,10 @@ quant_batched_kernel(const RowsArgs a) {
           if (weighted) block_weight(b, w);
         }
       }
-      finish_blocks(b, kb0, KB, gs, dst, sf_row, lane);
+      finish_blocks<kLoose && kSrc != kGather>(b, kb0, KB, gs, dst, sf_row, lane);
     }
   }
-  benign_fill_dead(a.counts, a.E, a.cap, n_rt, n_kt, a.sfb);
+  benign_fill_dead<kLoose>(a.counts, a.E, a.cap, n_rt, n_kt, a.sfb);
 }
 
 // n 16-byte words by one warp, eight of them per lane in flight.
@@ -337,7 +358,7 @@ scatter_fp4_rows_kernel(const uint8_t* __restrict__ q, long long q_pitch, const 
   LiveRows rows;
   rows.make(counts, E, cap, s_prefix);
   const unsigned nwarps = gridDim.x * kWarpsPerBlock;
-  const bool words = (KB % 4) == 0 && (sf_pitch % 4) == 0 && (reinterpret_cast<uintptr_t>(q_sf) % 4) == 0;
+  const bool words = (KB % 4) == 0 && (sf_pitch % 4) == 0 && ((reinterpret_cast<uintptr_t>(q_sf) | reinterpret_cast<uintptr_t>(sfb)) % 4) == 0;
   for (unsigned j = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); j < rows.total; j += nwarps) {
     int e, r;
     if (!rows.find(j, e, r)) continue;
@@ -354,7 +375,7 @@ scatter_fp4_rows_kernel(const uint8_t* __restrict__ q, long long q_pitch, const 
     }
     warp_copy(reinterpret_cast<const uint4*>(q + t * q_pitch), reinterpret_cast<uint4*>(b_act + slot * (K / 2)), K / 32, lane);
   }
-  benign_fill_dead(counts, E, cap, n_rt, n_kt, sfb);
+  benign_fill_dead<true>(counts, E, cap, n_rt, n_kt, sfb);
 }
 
 // quant_rows: token-order rows -> row-major codes and natural-order scales, one shared global scale.
@@ -485,8 +506,9 @@ template <int kSrc>
 int launch_batched(const RowsArgs& a, int sm_count, cudaStream_t s) {
   PNV_REQUIRE((long long)a.E * a.cap < (1LL << 31), "E * cap must fit int32");
   const long long units = (long long)a.E * a.cap * ceil_div_i(a.K / kSfBlock, 32);
-  PNV_CUDA(launch_pdl(quant_batched_kernel<kSrc>, dim3(grid_for(units, sm_count, kBatchedBlocks)), dim3(kThreads),
-                      live_rows_smem(a.E), s, pdl_enabled(), a));
+  const bool loose = (reinterpret_cast<uintptr_t>(a.b_act) | reinterpret_cast<uintptr_t>(a.sfb)) % 16 != 0;
+  PNV_CUDA(launch_pdl(loose ? quant_batched_kernel<kSrc, true> : quant_batched_kernel<kSrc, false>,
+                      dim3(grid_for(units, sm_count, kBatchedBlocks)), dim3(kThreads), live_rows_smem(a.E), s, pdl_enabled(), a));
   return PNV_OK;
 }
 
