@@ -150,6 +150,9 @@ extern "C" int pnv_compress(const uint8_t* w_packed, const uint8_t* w_blockscale
   PNV_REQUIRE(k > 0 && k % 8 == 0,
               "compress: K must be a multiple of 8 (whole 4-pair chunks), got %d", k);
   PNV_REQUIRE(reinterpret_cast<uintptr_t>(w_packed) % 4 == 0, "compress: the packed weights must be 4-byte aligned");
+  PNV_REQUIRE((reinterpret_cast<uintptr_t>(a_comp) | reinterpret_cast<uintptr_t>(sfa)) % 16 == 0 &&
+                  reinterpret_cast<uintptr_t>(e_meta) % 4 == 0,
+              "compress: a_comp and sfa must be 16-byte aligned, e_meta 4-byte aligned");
   cudaStream_t s = (cudaStream_t)stream;
   WeightDims wd = weight_dims(features, k);
   const long long tiles = (long long)experts * (wd.m_e / 128) * ceil_div_i(wd.k_e / 16, kTileLines);

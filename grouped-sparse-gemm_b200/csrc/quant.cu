@@ -491,6 +491,16 @@ int grid_for(long long warp_items, int sm_count, int per_sm = 8) {      // 8 x 2
   return (int)blocks;
 }
 
+bool aligned_to(const void* p, unsigned n) { return reinterpret_cast<uintptr_t>(p) % n == 0; }
+
+// What the row kernels' vector accesses need of their pointers (a bf16 source is read 16 bytes at a time).
+int check_alignment(const void* x, const uint8_t* b_act, unsigned b_align, const uint8_t* sfb) {
+  PNV_REQUIRE(aligned_to(x, 16), "the bf16 source must be 16-byte aligned");
+  PNV_REQUIRE(aligned_to(b_act, b_align), "the codes must be %u-byte aligned", b_align);
+  PNV_REQUIRE(aligned_to(sfb, 4), "the scales must be 4-byte aligned");
+  return PNV_OK;
+}
+
 int check_common(const void* x, const float* gscale, const int32_t* counts, int E, int rows, int K,
                  const uint8_t* b_act, const uint8_t* sfb, const char* kname) {
   PNV_REQUIRE(x && gscale && counts && b_act && sfb, "null pointer argument");
@@ -504,9 +514,10 @@ int check_common(const void* x, const float* gscale, const int32_t* counts, int 
 // One launch of the shared kernel: at most a wave of warps, one per 32 K-blocks of a row of the capacity.
 template <int kSrc>
 int launch_batched(const RowsArgs& a, int sm_count, cudaStream_t s) {
+  if (int rc = check_alignment(a.x, a.b_act, kSrc == kGather ? 16 : 8, a.sfb)) return rc;
   PNV_REQUIRE((long long)a.E * a.cap < (1LL << 31), "E * cap must fit int32");
   const long long units = (long long)a.E * a.cap * ceil_div_i(a.K / kSfBlock, 32);
-  const bool loose = (reinterpret_cast<uintptr_t>(a.b_act) | reinterpret_cast<uintptr_t>(a.sfb)) % 16 != 0;
+  const bool loose = !aligned_to(a.b_act, 16) || !aligned_to(a.sfb, 16);
   PNV_CUDA(launch_pdl(loose ? quant_batched_kernel<kSrc, true> : quant_batched_kernel<kSrc, false>,
                       dim3(grid_for(units, sm_count, kBatchedBlocks)), dim3(kThreads), live_rows_smem(a.E), s, pdl_enabled(), a));
   return PNV_OK;
@@ -567,6 +578,8 @@ extern "C" int pnv_scatter_quant_act(const void* a1, const int64_t* flat_tok,
   if (int rc = check_common(a1 ? a1 : (const void*)&dummy, gscale, &dummy, experts, cap, k, b_act, sfb, "K"))
     return rc;
   PNV_REQUIRE(n_routes == 0 || a1, "null pointer argument");
+  if (n_routes > 0)
+    if (int rc = check_alignment(a1, b_act, 16, sfb)) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   PNV_CUDA(cudaMemsetAsync(sfb, kBenignSf, (size_t)sf_numel(cap, k, experts), s));
   if (n_routes == 0) return PNV_OK;
@@ -585,6 +598,7 @@ extern "C" int pnv_gated_act(const void* x2, int64_t rows, int n, int interleave
   PNV_REQUIRE(x2 && y, "null pointer argument");
   PNV_REQUIRE(n > 0 && n % kSfBlock == 0, "intermediate width N must be a multiple of %d, got %d", kSfBlock, n);
   if (rows <= 0) return PNV_OK;
+  PNV_REQUIRE(aligned_to(x2, 16) && aligned_to(y, 16), "gated_act buffers must be 16-byte aligned");
   long long total = rows * (n / 8);
   long long blocks = (total + kThreads - 1) / kThreads;
   if (blocks > 148LL * 32) blocks = 148LL * 32;
@@ -613,6 +627,8 @@ extern "C" int pnv_quant_rows(const void* x, const float* gscale, int64_t tokens
   if (tokens == 0) return PNV_OK;
   PNV_REQUIRE(x && gscale && q && q_sf, "null pointer argument");
   PNV_REQUIRE(tokens < (1LL << 31), "too many tokens");
+  PNV_REQUIRE(aligned_to(x, 16) && aligned_to(q, 16), "quant_rows: the bf16 rows and the codes must be 16-byte aligned");
+  PNV_REQUIRE((k / kSfBlock) % 4 != 0 || aligned_to(q_sf, 4), "quant_rows: the scales must be 4-byte aligned");
   PNV_CUDA(launch_pdl(quant_rows_kernel, dim3(grid_for(tokens, sm_count)), dim3(kThreads), 0, (cudaStream_t)stream,
                       pdl_enabled(), (const __nv_bfloat16*)x, gscale, (unsigned)tokens, k, q, q_sf));
   return PNV_OK;

@@ -474,6 +474,8 @@ extern "C" int pnv_moe_finalize(void* out, const void* fused, const int32_t* rou
   if (tokens == 0) return PNV_OK;
   PNV_REQUIRE(out && fused && route_dest, "null pointer argument");
   PNV_REQUIRE(tokens < (1LL << 31), "too many tokens");
+  PNV_REQUIRE((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(fused)) % 16 == 0,
+              "moe_finalize buffers must be 16-byte aligned");
   const int vecs = k / 8;
   cudaStream_t s = (cudaStream_t)stream;
   const bool pdl = pdl_enabled();

@@ -9,6 +9,11 @@
  * Return value: 0 on success, a PNV_ERR_* code otherwise; pnv_last_error() then returns a
  * NUL-terminated description (thread-local, valid until the next failing call on that thread).
  *
+ * Alignment: every pointer to the alignment of its element type.  bf16 buffers, packed codes and compressed weights to 16
+ * bytes, scale buffers to 4, beyond that where a comment says so.  Exceptions: the packed weights of pnv_compress 4 bytes,
+ * its scales any; the codes of pnv_quant_act and pnv_silu_mul_quant_act 8 bytes; the weight and scale operands of
+ * group_mm, and the scales that pnv_pack_wire_rows reads when k is a multiple of 512, 16 bytes.  A pointer that the kernels cannot take is refused with PNV_ERR_INVALID_ARGUMENT.
+ *
  * Each declaration names the interface of the reference project (IST-DASLab/grouped-sparse-GEMM,
  * paths relative to its root) that it stands in for.
  */
