@@ -29,14 +29,15 @@ __device__ __forceinline__ uint32_t gather_sf_word(uint32_t my_byte) {
          (__shfl_down_sync(0xffffffffu, my_byte, 2) << 16) | (__shfl_down_sync(0xffffffffu, my_byte, 3) << 24);
 }
 
-// One 32-element block in one lane: 64 bytes in, two bf16 to a register.  `wide`: the source is 32-byte aligned.
+// One 32-element block in one lane: 64 bytes in, two bf16 to a register.  `wide`: the source is 32-byte aligned.  (The load
+// is volatile with a memory clobber so that the compiler keeps it behind pdl_wait().)
 struct BlockRegs {
   uint32_t lo[8], hi[8];
 };
 __device__ __forceinline__ void load32(const uint8_t* src, bool wide, uint32_t (&w)[8]) {
   if (wide) {
-    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(src));
+    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(src) : "memory");
   } else {
     const uint4 v0 = __ldg(reinterpret_cast<const uint4*>(src)), v1 = __ldg(reinterpret_cast<const uint4*>(src) + 1);
     w[0] = v0.x; w[1] = v0.y; w[2] = v0.z; w[3] = v0.w;
