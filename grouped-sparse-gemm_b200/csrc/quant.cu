@@ -168,43 +168,44 @@ __device__ __forceinline__ void benign_fill_dead(const int* __restrict__ counts,
 // The live rows of a batched operand, numbered expert after expert.  make() builds the prefix sums of the clamped
 // counts - up to 32 experts every warp in its own registers, without a barrier; up to kMaxPrefixExperts the block in
 // shared memory - and find() turns a row's number into its slot.  With more experts there are no prefix sums: every slot is
-// a row and the dead ones are skipped.  All lanes of a warp ask for the same row.
+// a row and the dead ones are skipped.  All lanes of a warp ask for the same row.  Row numbers are unsigned 32-bit: K = 32
+// leaves room for more than 2^31 rows in this GPU's memory.
 constexpr int kMaxPrefixExperts = 8192;
 struct LiveRows {
   const int* counts;
   int E, cap;
-  int* prefix;           // shared memory, [E + 1]
-  int lane_first;        // up to 32 experts: first row of expert `lane` (INT_MAX past the last)
+  unsigned* prefix;      // shared memory, [E + 1]
+  unsigned lane_first;   // up to 32 experts: first row of expert `lane` (the largest number past the last)
   unsigned total;
-  __device__ __forceinline__ void make(const int* counts_, int E_, int cap_, int* smem) {
+  __device__ __forceinline__ void make(const int* counts_, int E_, int cap_, unsigned* smem) {
     counts = counts_; E = E_; cap = cap_; prefix = smem; lane_first = 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (E > kMaxPrefixExperts) { total = (unsigned)E * (unsigned)cap; return; }
     if (E <= 32) {
-      const int c = lane < E ? max(0, min(counts[lane], cap)) : 0;
-      int v = c;
+      const unsigned c = lane < E ? (unsigned)max(0, min(counts[lane], cap)) : 0u;
+      unsigned v = c;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        const unsigned u = __shfl_up_sync(0xffffffffu, v, o);
         if (lane >= o) v += u;
       }
-      lane_first = lane < E ? v - c : 0x7FFFFFFF;
-      total = (unsigned)__shfl_sync(0xffffffffu, v, 31);
+      lane_first = lane < E ? v - c : 0xFFFFFFFFu;
+      total = __shfl_sync(0xffffffffu, v, 31);
       return;
     }
-    __shared__ int s_warp[kWarpsPerBlock];
-    int carry = 0;
+    __shared__ unsigned s_warp[kWarpsPerBlock];
+    unsigned carry = 0;
     for (int e0 = 0; e0 < E; e0 += kThreads) {
       const int e = e0 + (int)threadIdx.x;
-      int v = e < E ? max(0, min(counts[e], cap)) : 0;
+      unsigned v = e < E ? (unsigned)max(0, min(counts[e], cap)) : 0u;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        const unsigned u = __shfl_up_sync(0xffffffffu, v, o);
         if (lane >= o) v += u;
       }
       if (lane == 31) s_warp[warp] = v;
       __syncthreads();
-      int before = carry, sum = 0;
+      unsigned before = carry, sum = 0;
 #pragma unroll
       for (int i = 0; i < kWarpsPerBlock; ++i) {
         if (i < warp) before += s_warp[i];
@@ -216,13 +217,13 @@ struct LiveRows {
     }
     if (threadIdx.x == 0) smem[0] = 0;
     __syncthreads();
-    total = (unsigned)carry;
+    total = carry;
   }
   // row number j < total -> expert and row of the expert; false for a dead slot (only without prefix sums)
   __device__ __forceinline__ bool find(unsigned j, int& e, int& r) const {
     if (E <= 32) {       // the last expert whose first row is at or before j
-      e = 31 - __clz(__ballot_sync(0xffffffffu, (unsigned)lane_first <= j));
-      r = (int)j - __shfl_sync(0xffffffffu, lane_first, e);
+      e = 31 - __clz(__ballot_sync(0xffffffffu, lane_first <= j));
+      r = (int)(j - __shfl_sync(0xffffffffu, lane_first, e));
       return true;
     }
     if (E > kMaxPrefixExperts) {
@@ -233,11 +234,11 @@ struct LiveRows {
     int lo = 0, hi = E - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      if ((unsigned)prefix[mid] <= j) lo = mid;
+      if (prefix[mid] <= j) lo = mid;
       else hi = mid - 1;
     }
     e = lo;
-    r = (int)j - prefix[lo];
+    r = (int)(j - prefix[lo]);
     return true;
   }
 };
@@ -265,7 +266,7 @@ constexpr int kBatchedBlocks = 4;
 template <int kSrc, bool kLoose>
 __global__ void __launch_bounds__(kThreads, kBatchedBlocks)
 quant_batched_kernel(const RowsArgs a) {
-  extern __shared__ int s_prefix[];
+  extern __shared__ unsigned s_prefix[];
   pdl_wait();
   pdl_launch_dependents();
   const int KB = a.K / kSfBlock;
@@ -280,7 +281,7 @@ quant_batched_kernel(const RowsArgs a) {
   // piece.  (Consecutive warps take consecutive rows of one piece; the scale words of 32 rows share lines.)
   unsigned pieces = 1;
   int piece_blocks = KB;
-  if (rows.total > 0 && 2u * rows.total <= nwarps && KB > 32) {
+  if (rows.total > 0 && rows.total <= nwarps / 2u && KB > 32) {
     pieces = min(nwarps / rows.total, (unsigned)(KB + 31) / 32u);
     piece_blocks = (int)(((unsigned)KB + pieces - 1) / pieces + 31) / 32 * 32;
     pieces = (unsigned)(KB + piece_blocks - 1) / (unsigned)piece_blocks;
@@ -349,7 +350,7 @@ __global__ void __launch_bounds__(kThreads)
 scatter_fp4_rows_kernel(const uint8_t* __restrict__ q, long long q_pitch, const uint8_t* __restrict__ q_sf,
                         long long sf_pitch, const int* __restrict__ src_tok, const int* __restrict__ counts, int K, int E,
                         int cap, uint8_t* __restrict__ b_act, uint8_t* __restrict__ sfb) {
-  extern __shared__ int s_prefix[];
+  extern __shared__ unsigned s_prefix[];
   pdl_wait();
   pdl_launch_dependents();
   const int KB = K / kSfBlock;
@@ -516,7 +517,9 @@ int check_common(const void* x, const float* gscale, const int32_t* counts, int 
 template <int kSrc>
 int launch_batched(const RowsArgs& a, int sm_count, cudaStream_t s) {
   if (int rc = check_alignment(a.x, a.b_act, kSrc == kGather ? 16 : 8, a.sfb)) return rc;
-  PNV_REQUIRE((long long)a.E * a.cap < (1LL << 31), "E * cap must fit int32");
+  if (kSrc == kGather) PNV_REQUIRE((long long)a.E * a.cap < (1LL << 31), "E * cap must fit int32");
+  // (a grid stride short of 2^32, so that a warp's next row number cannot wrap around)
+  PNV_REQUIRE((long long)a.E * a.cap < (1LL << 32) - (1LL << 24), "experts * max_n must be below 2^32 - 2^24");
   const long long units = (long long)a.E * a.cap * ceil_div_i(a.K / kSfBlock, 32);
   const bool loose = !aligned_to(a.b_act, 16) || !aligned_to(a.sfb, 16);
   PNV_CUDA(launch_pdl(loose ? quant_batched_kernel<kSrc, true> : quant_batched_kernel<kSrc, false>,

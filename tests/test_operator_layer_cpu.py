@@ -23,3 +23,15 @@ def test_only_ops_without_float_results_pass_autograd_by(pnk):
 
     assert [op for op in FLOAT_RESULTS if has_autograd_kernel(op)] == []
     assert [op for op in INTEGER_OR_NO_RESULTS if not has_autograd_kernel(op)] == []
+
+
+@pytest.mark.skipif(torch.cuda.is_available(), reason="the call would be launched; its pointers stand for nothing")
+def test_quantizers_take_more_than_two_to_the_31_rows(pnk):
+    """E * max_n of 2^31 and beyond fits this GPU's memory at K = 32 (64 + 16 + 4 bytes a row): refused neither by the
+    argument checks nor by a 32-bit row number.  (Without a device the launch itself fails, with another code.)"""
+    from paired_nvfp4_kernels import _cabi
+    p = 0x100000
+    rc = _cabi.lib.pnv_quant_act(p, p, 0, p, 2, 1 << 30, 32, p, p, 148, None)
+    assert rc == 2, _cabi.lib.pnv_last_error()
+    rc = _cabi.lib.pnv_quant_act(p, p, 0, p, 4, (1 << 30) - 1, 32, p, p, 148, None)
+    assert rc == 1 and b"2^32" in _cabi.lib.pnv_last_error()
