@@ -63,7 +63,12 @@ void check_arch(const Tensor& t) {
 
 cudaStream_t current_stream(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
+// An uninitialised tensor.  Through the dispatcher only where torch is to fill uninitialised memory
+// (torch.use_deterministic_algorithms): rows past an expert's count then hold the same bytes in every run.
 Tensor empty_on(const Tensor& like, at::IntArrayRef sizes, at::ScalarType dtype) {
+  const at::Context& ctx = at::globalContext();
+  if (C10_UNLIKELY(ctx.deterministicAlgorithms() && ctx.deterministicFillUninitializedMemory()))
+    return at::empty(sizes, like.options().dtype(dtype));
   return at::detail::empty_cuda(sizes, dtype, like.device(), c10::nullopt);
 }
 

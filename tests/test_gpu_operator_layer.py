@@ -33,6 +33,25 @@ def test_float_results_say_that_they_have_no_backward(ops, op):
     assert not q.requires_grad
 
 
+def test_uninitialised_rows_are_filled_where_torch_fills_them(ops):
+    """Under torch.use_deterministic_algorithms the bytes that no kernel writes are torch's fill value, as for torch.empty."""
+    counts = dev(np.array([2, 0, 5], np.int32))
+    x = torch.randn((3, 5, 64), device="cuda").to(torch.bfloat16)
+    ids = dev(np.array([[0, 2], [0, 2], [2, 2], [2, 2]], np.int64))
+    before = torch.are_deterministic_algorithms_enabled(), torch.is_deterministic_algorithms_warn_only_enabled()
+    torch.use_deterministic_algorithms(True)
+    try:
+        b, _ = ops.quant_act(x, torch.ones(1, device="cuda"), counts, 128)
+        plan_counts, _, src_tok, src_route = ops.dispatch_plan(ids, 0, 3, 8)
+    finally:
+        torch.use_deterministic_algorithms(before[0], warn_only=before[1])
+    assert bool((b[0, 2:] == 255).all()) and bool((b[1] == 255).all())
+    dead = torch.arange(8, device="cuda")[None, :] >= plan_counts[:, None]
+    assert plan_counts.tolist() == [2, 0, 6]
+    for t in (src_tok, src_route):
+        assert bool((t.view(3, 8)[dead] == torch.iinfo(torch.int32).max).all())
+
+
 # ---- split-K workspaces ------------------------------------------------------------------------------------------
 
 K_SPLIT = 3584         # seven K stages of 512
