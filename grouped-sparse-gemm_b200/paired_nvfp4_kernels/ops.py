@@ -9,6 +9,7 @@ import torch
 from . import _cabi
 
 _lib = _cabi.lib
+SF_BLOCK = 32          # dense K elements per scale
 TORCH_LIB_PATH = os.path.join(os.path.dirname(_cabi.LIB_PATH), "libpaired_nvfp4_torch.so")
 
 

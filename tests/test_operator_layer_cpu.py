@@ -35,3 +35,16 @@ def test_quantizers_take_more_than_two_to_the_31_rows(pnk):
     assert rc == 2, _cabi.lib.pnv_last_error()
     rc = _cabi.lib.pnv_quant_act(p, p, 0, p, 4, (1 << 30) - 1, 32, p, p, 148, None)
     assert rc == 1 and b"2^32" in _cabi.lib.pnv_last_error()
+
+
+def test_names_of_the_ops_module(pnk):
+    """Everything a program could take from paired_nvfp4_kernels.ops: the operators under their own names, the helpers, the
+    block size of the scales."""
+    from paired_nvfp4_kernels import ops
+    assert ops.SF_BLOCK == 32
+    for name in INTEGER_OR_NO_RESULTS + FLOAT_RESULTS + [
+            "group_mm_configs", "group_mm_swiglu_configs", "set_sm_margin", "wire_row_bytes", "wire_expert_ids",
+            "set_silu_table", "group_mm_device_status"]:
+        assert callable(getattr(ops, name)), name
+    with pytest.raises(AttributeError):
+        ops.no_such_operator
