@@ -7,8 +7,10 @@ Both land in grouped-sparse-gemm_b200/paired_nvfp4_kernels/, next to the Python 
 that loads them.  PAIRED_NVFP4_PTXAS_V=1 (or --ptxas-v) prints registers / spills / shared memory.
 """
 import os
+import runpy
 import subprocess
 import sys
+from importlib.util import find_spec
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -53,8 +55,23 @@ def build(force=False, ptxas_v=False, verbose=True):
     return OUT
 
 
+def torch_build_id():
+    """Which torch an operator layer built now belongs to (read without importing torch).  C++ against torch's headers
+    loads into that build alone."""
+    version = runpy.run_path(os.path.join(os.path.dirname(find_spec("torch").origin), "version.py"))
+    return f"torch-build:{version['__version__']}:{version.get('git_version')};"
+
+
+def torch_ops_up_to_date():
+    """Newer than its sources, and built for the torch that is installed: the library carries the id."""
+    if not up_to_date(TORCH_OUT, [TORCH_SRC, HEADER]):
+        return False
+    with open(TORCH_OUT, "rb") as f:
+        return torch_build_id().encode() in f.read()
+
+
 def build_torch_ops(force=False, verbose=True):
-    if not force and up_to_date(TORCH_OUT, [TORCH_SRC, HEADER]):
+    if not force and torch_ops_up_to_date():
         return TORCH_OUT
     import torch
     root = os.path.dirname(torch.__file__)
@@ -62,7 +79,7 @@ def build_torch_ops(force=False, verbose=True):
     # the g++ on PATH, not $CXX: libstdc++ has to be the shared one that torch uses (a second, static copy inside this
     # library crashed while formatting an error message)
     _run(["g++", "-shared", "-fPIC", "-std=c++17", "-O2", "-fvisibility=hidden",
-          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DPNV_TORCH_BUILD_ID="{torch_build_id()}"',
           "-isystem", os.path.join(root, "include"), "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"),
           "-isystem", os.path.join(_cuda_home(), "include"), TORCH_SRC, "-o", TORCH_OUT,
           "-L" + lib, "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10",

@@ -650,6 +650,9 @@ std::vector<std::string> group_mm_swiglu_configs() {      // csrc/ops.cu:585-589
 // Leave `n` SMs out of every persistent launch (see paired_nvfp4_kernels.ops.set_sm_margin).
 extern "C" __attribute__((visibility("default"))) void pnv_torch_set_sm_margin(int n) { g_sm_margin.store(std::max(0, n)); }
 
+// The torch this library was built for, looked up in the file by build.py.
+extern "C" __attribute__((visibility("default"))) const char* pnv_torch_build_id() { return PNV_TORCH_BUILD_ID; }
+
 #define PNV_GEMM_OPERANDS "Tensor a_comp, Tensor e_meta, Tensor sfa, Tensor b_act, Tensor sfb, Tensor alphas, Tensor expert_num_tokens, "
 // the defaults are paired_nvfp4_kernels.DEFAULT_TACTIC
 #define PNV_TACTIC "int config_id=0, int cluster_m=2, int cluster_n=1"

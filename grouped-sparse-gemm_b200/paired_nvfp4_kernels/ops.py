@@ -21,7 +21,8 @@ def _load():
         torch.ops.load_library(TORCH_LIB_PATH)
         lib = ctypes.CDLL(TORCH_LIB_PATH)
     except OSError as exc:  # pragma: no cover
-        raise ImportError(f"could not load {TORCH_LIB_PATH}: {exc}") from exc
+        raise ImportError(f"could not load {TORCH_LIB_PATH}: {exc} (it loads into the torch it was built for: after a change of "
+                          "torch run `python grouped-sparse-gemm_b200/build.py`)") from exc
     lib.pnv_torch_set_sm_margin.argtypes = [ctypes.c_int]
     lib.pnv_torch_set_sm_margin.restype = None
     return lib

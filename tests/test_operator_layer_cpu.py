@@ -1,4 +1,7 @@
 """No-GPU checks of the operator layer and of its build."""
+import importlib.util
+import os
+
 import pytest
 import torch
 
@@ -48,3 +51,15 @@ def test_names_of_the_ops_module(pnk):
         assert callable(getattr(ops, name)), name
     with pytest.raises(AttributeError):
         ops.no_such_operator
+
+
+def test_the_operator_library_is_rebuilt_for_another_torch(pnk, monkeypatch):
+    """C++ against torch's headers does not load into another torch, whatever the files' times say."""
+    path = os.path.join(os.path.dirname(os.path.dirname(pnk.__file__)), "build.py")
+    spec = importlib.util.spec_from_file_location("pnv_build", path)
+    build = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(build)
+    assert torch.__version__ in build.torch_build_id() and torch.version.git_version in build.torch_build_id()
+    assert build.torch_ops_up_to_date()
+    monkeypatch.setattr(build, "torch_build_id", lambda: "torch-build:0.0:none;")
+    assert not build.torch_ops_up_to_date()
