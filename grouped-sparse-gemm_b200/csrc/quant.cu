@@ -1,12 +1,14 @@
 // Activation quantizers: bf16 -> e2m1 codes + one UE4M3 scale per 32 elements, written straight
 // into the grouped GEMM's B-operand layouts (row-major codes, swizzled scale atoms).
 //
-// quant_act, silu_mul_quant_act and scatter_quant_act_planned share one kernel.  Its units are the live rows (r < counts[e])
-// of the batched operand, found through a prefix sum of counts that every block makes for itself, so that skewed or mostly
-// empty capacities cost nothing: a warp takes a row, or a piece of one where there are fewer rows than warps, 32 K-blocks
-// at a time with one whole block per lane (64 bytes in, or 128 with gate and up; 16 bytes of codes out; the scale step,
-// with its two IEEE divisions, once per block).  The bytes of the scale buffer that no live row writes become 0x38 in the
-// same kernel, a 16-byte line per thread.
+// quant_act, silu_mul_quant_act and scatter_quant_act_planned share two kernels.  Their work is the live rows
+// (r < counts[e]) of the batched operand, found through a prefix sum of counts that every block makes for itself, so that
+// skewed or mostly empty capacities cost nothing.  One whole 32-element K-block per lane (64 bytes in, or 128 with gate and
+// up; 16 bytes of codes out; the scale step, with its two IEEE divisions, once per block).  With long rows
+// (quant_batched_kernel) a warp takes a row, or a piece of one where there are fewer rows than warps, 32 K-blocks at a
+// time; otherwise (quant_quads_kernel) the rows' K-blocks are laid end to end and dealt four by four, so that short rows
+// and remainders leave no lane idle.  The bytes of the scale buffer that no live row writes become 0x38 in the same kernel,
+// a 16-byte line per thread.
 // Bound: HBM for plain rows (131072 rows of 2048: 118 us, 687 MB), issue slots (0.68 of them used) and L2 for gathered
 // ones (102 us; 150 MB written, the rows read from L2 eight times over), the special-function unit and issue for SiTU.
 // Loads are 32 bytes a lane where the input is aligned to that: 16-byte loads at a stride of 64 bytes take twice the
@@ -56,6 +58,14 @@ __device__ __forceinline__ uint4 block_codes(const BlockRegs& b, float inv) {
   return make_uint4(quant8_packed(b.lo[0], b.lo[1], b.lo[2], b.lo[3], inv), quant8_packed(b.lo[4], b.lo[5], b.lo[6], b.lo[7], inv),
                     quant8_packed(b.hi[0], b.hi[1], b.hi[2], b.hi[3], inv), quant8_packed(b.hi[4], b.hi[5], b.hi[6], b.hi[7], inv));
 }
+__device__ __forceinline__ void store_codes(uint4* dst, const uint4& codes, bool dst16) {      // 8-byte aligned otherwise
+  if (dst16) {
+    *dst = codes;
+  } else {
+    reinterpret_cast<uint2*>(dst)[0] = make_uint2(codes.x, codes.y);
+    reinterpret_cast<uint2*>(dst)[1] = make_uint2(codes.z, codes.w);
+  }
+}
 // Every value times the bf16 weight w, rounded to bf16 (the product of two bf16 numbers is exact in float, so the packed
 // multiplication rounds like the float product rounded to bf16).
 __device__ __forceinline__ void block_weight(BlockRegs& b, float w) {
@@ -74,8 +84,7 @@ __device__ __forceinline__ void block_weight(BlockRegs& b, float w) {
 enum RowSource : int { kPlain = 0, kGated = 1, kGather = 2 };
 
 // 32 K-blocks from kb0 on, one per lane in b, are scaled, rounded and stored; a row's four scales of one 128-K group are one
-// aligned word of the swizzled layout.  KB: the blocks of the whole row.  kLoose: the codes are 8-byte aligned only.
-template <bool kLoose = false>
+// aligned word of the swizzled layout.  KB: the blocks of the whole row.
 __device__ __forceinline__ void finish_blocks(const BlockRegs& b, int kb0, int KB, float gs, uint4* __restrict__ dst,
                                               uint8_t* __restrict__ sf_row, int lane) {
   const int kb = kb0 + lane;
@@ -83,14 +92,7 @@ __device__ __forceinline__ void finish_blocks(const BlockRegs& b, int kb0, int K
   if (kb < KB) {
     float inv;
     block_scale(block_amax(b), gs, sf_byte, inv);
-    const uint4 codes = block_codes(b, inv);
-    if constexpr (!kLoose) {
-      dst[kb] = codes;
-    } else {
-      uint2* half = reinterpret_cast<uint2*>(dst + kb);
-      half[0] = make_uint2(codes.x, codes.y);
-      half[1] = make_uint2(codes.z, codes.w);
-    }
+    dst[kb] = block_codes(b, inv);
   }
   const uint32_t word = gather_sf_word(sf_byte);
   if ((lane & 3) == 0 && kb < KB) *reinterpret_cast<uint32_t*>(sf_row + (kb >> 2) * 512) = word;
@@ -241,6 +243,31 @@ struct LiveRows {
     r = (int)(j - prefix[lo]);
     return true;
   }
+  // The same for a row of each lane's own (all lanes take part); a dead slot's expert is -1.
+  __device__ __forceinline__ void find_each(unsigned j, int& e, int& r) const {
+    int lo = 0;
+    if (E <= 32) {
+#pragma unroll
+      for (int step = 16; step > 0; step >>= 1) {
+        const unsigned first = __shfl_sync(0xffffffffu, lane_first, lo + step);      // (lo + step < 32)
+        if (first <= j) lo += step;
+      }
+      r = (int)(j - __shfl_sync(0xffffffffu, lane_first, lo));
+    } else if (E > kMaxPrefixExperts) {
+      lo = (int)(j / (unsigned)cap);
+      r = (int)(j - (unsigned)lo * (unsigned)cap);
+      if (lo >= E || r >= counts[lo]) lo = -1;
+    } else {
+      int hi = E - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (prefix[mid] <= j) lo = mid;
+        else hi = mid - 1;
+      }
+      r = (int)(j - prefix[lo]);
+    }
+    e = lo;
+  }
 };
 size_t live_rows_smem(int E) { return E <= 32 || E > kMaxPrefixExperts ? 0 : sizeof(int) * (size_t)(E + 1); }
 
@@ -261,9 +288,8 @@ struct RowsArgs {
 // next step's loads ahead of the arithmetic are 15 % slower.  The grid is one wave of them.
 constexpr int kBatchedBlocks = 4;
 
-// kLoose: codes or scales that are less than 16-byte aligned (pieces of a caller's larger buffer).  A form of its own,
-// because with the tests at run time the activation's form spilled and ran 1 % longer.
-template <int kSrc, bool kLoose>
+// A warp takes a row, or a piece of one: for rows of many K-blocks, 16-byte aligned destinations.
+template <int kSrc>
 __global__ void __launch_bounds__(kThreads, kBatchedBlocks)
 quant_batched_kernel(const RowsArgs a) {
   extern __shared__ unsigned s_prefix[];
@@ -322,10 +348,108 @@ quant_batched_kernel(const RowsArgs a) {
           if (weighted) block_weight(b, w);
         }
       }
-      finish_blocks<kLoose && kSrc != kGather>(b, kb0, KB, gs, dst, sf_row, lane);
+      finish_blocks(b, kb0, KB, gs, dst, sf_row, lane);
     }
   }
-  benign_fill_dead<kLoose>(a.counts, a.E, a.cap, n_rt, n_kt, a.sfb);
+  benign_fill_dead<false>(a.counts, a.E, a.cap, n_rt, n_kt, a.sfb);
+}
+
+// The same for short rows, rows that leave many lanes of a warp's last 32 K-blocks idle, and destinations that are less
+// than 16-byte aligned (pieces of a caller's larger buffer).  The work is the quads of the live rows laid end to end - a
+// quad is four K-blocks, one word of scales, four lanes - cut into one range per warp, so that no lane idles whatever the
+// row length.  A warp looks up 32 rows at a time, one per lane, and its quads fetch theirs by shuffles: with short rows a
+// search per row is a chain of shared-memory reads in front of every few loads.
+template <int kSrc>
+__global__ void __launch_bounds__(kThreads, kBatchedBlocks)
+quant_quads_kernel(const RowsArgs a) {
+  extern __shared__ unsigned s_prefix[];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int KB = a.K / kSfBlock;
+  const int n_rt = sf_row_atoms(a.cap);
+  const int n_kt = sf_k_atoms(a.K);
+  const bool wide = (reinterpret_cast<uintptr_t>(a.x) & 31) == 0;
+  const bool dst16 = (reinterpret_cast<uintptr_t>(a.b_act) & 15) == 0;
+  const int lane = threadIdx.x & 31;
+  LiveRows rows;
+  rows.make(a.counts, a.E, a.cap, s_prefix);
+  const unsigned long long quads = (unsigned long long)rows.total * (unsigned)n_kt;
+  const unsigned nwarps = gridDim.x * kWarpsPerBlock;
+  const unsigned long long per_warp = (quads + 8ull * nwarps - 1) / (8ull * nwarps) * 8;
+  const unsigned long long q0 = per_warp * ((threadIdx.x >> 5) * gridDim.x + blockIdx.x);      // (few ranges: on many SMs)
+  if (q0 < quads) {
+    int left = (int)min(per_warp, quads - q0) - (lane >> 2);       // quads of the range from this lane's on
+    unsigned row0 = (unsigned)(q0 / (unsigned)n_kt);               // first row looked up
+    const int kt0 = (int)(q0 - (unsigned long long)row0 * (unsigned)n_kt) + (lane >> 2);
+    int b = kt0 / n_kt, kt = kt0 - b * n_kt;                       // this lane's quad: row row0 + b, K-blocks 4 kt ...
+    const int step_b = 8 / n_kt, step_kt = 8 - step_b * n_kt;
+    const long long row_bytes = (kSrc == kGated ? 4LL : 2LL) * a.K;
+    const bool weighted = kSrc == kGather && a.topk_w != nullptr;
+    unsigned my_slot = 0;                                          // of row row0 + lane
+    int my_e = 0, my_tok = 0;
+    float my_w = 1.f;
+    bool look = true;
+    while (__any_sync(0xffffffffu, left > 0)) {
+      if (!look && __any_sync(0xffffffffu, b > 31)) {              // on to the next rows: the first quad's becomes row0
+        const int shift = __shfl_sync(0xffffffffu, b, 0);
+        row0 += (unsigned)shift;
+        b -= shift;
+        look = true;
+      }
+      if (look) {
+        look = false;
+        const unsigned j = min(row0 + (unsigned)lane, rows.total - 1u);
+        int r;
+        rows.find_each(j, my_e, r);
+        my_slot = my_e < 0 ? 0u : (unsigned)my_e * (unsigned)a.cap + (unsigned)r;
+        if constexpr (kSrc == kGather) {
+          if (my_e >= 0) {
+            my_tok = a.src_tok[my_slot];
+            if (weighted) my_w = __bfloat162float(__float2bfloat16_rn(a.topk_w[a.src_route[my_slot]]));
+          }
+        }
+      }
+      const int e = __shfl_sync(0xffffffffu, my_e, b);
+      const unsigned slot = __shfl_sync(0xffffffffu, my_slot, b);
+      long long src_row = slot;
+      float w = 1.f;
+      if constexpr (kSrc == kGather) {
+        src_row = __shfl_sync(0xffffffffu, my_tok, b);
+        if (weighted) w = __shfl_sync(0xffffffffu, my_w, b);
+      }
+      const bool on = left > 0 && e >= 0;
+      const int kb = kt * 4 + (lane & 3);
+      uint32_t sf_byte = kBenignSf;   // blocks past K keep the benign byte in the layout's slop
+      if (on && kb < KB) {
+        const float gs = a.gscale[a.gscale_per_expert ? e : 0];
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(a.x) + src_row * row_bytes;
+        BlockRegs blk;
+        if constexpr (kSrc == kGated) {
+          const uint8_t* gate = src + (a.interleaved ? 128LL : 64LL) * kb;
+          const uint8_t* up = a.interleaved ? gate + 64 : gate + 64LL * KB;
+          BlockRegs g, up_b;
+          load_block(gate, wide, g);
+          load_block(up, wide, up_b);
+          gated_act16(g.lo, up_b.lo, a.act, blk.lo);
+          gated_act16(g.hi, up_b.hi, a.act, blk.hi);
+        } else {
+          load_block(src + 64LL * kb, wide, blk);
+          if (weighted) block_weight(blk, w);
+        }
+        float inv;
+        block_scale(block_amax(blk), gs, sf_byte, inv);
+        store_codes(reinterpret_cast<uint4*>(a.b_act + (long long)slot * (a.K / 2)) + kb, block_codes(blk, inv), dst16);
+      }
+      const uint32_t word = gather_sf_word(sf_byte);
+      if (on && (lane & 3) == 0)
+        *reinterpret_cast<uint32_t*>(a.sfb + sf_offset(e, (int)(slot - (unsigned)e * (unsigned)a.cap), kt * 4, n_rt, n_kt)) = word;
+      left -= 8;
+      b += step_b;
+      kt += step_kt;
+      if (kt >= n_kt) { kt -= n_kt; ++b; }
+    }
+  }
+  benign_fill_dead<true>(a.counts, a.E, a.cap, n_rt, n_kt, a.sfb);
 }
 
 // n 16-byte words by one warp, eight of them per lane in flight.
@@ -513,16 +637,19 @@ int check_common(const void* x, const float* gscale, const int32_t* counts, int 
   return PNV_OK;
 }
 
-// One launch of the shared kernel: at most a wave of warps, one per 32 K-blocks of a row of the capacity.
+// One launch of the shared kernel: at most a wave of warps, one per 32 K-blocks of a row of the capacity (or eight quads).
 template <int kSrc>
 int launch_batched(const RowsArgs& a, int sm_count, cudaStream_t s) {
   if (int rc = check_alignment(a.x, a.b_act, kSrc == kGather ? 16 : 8, a.sfb)) return rc;
   if (kSrc == kGather) PNV_REQUIRE((long long)a.E * a.cap < (1LL << 31), "E * cap must fit int32");
   // (a grid stride short of 2^32, so that a warp's next row number cannot wrap around)
   PNV_REQUIRE((long long)a.E * a.cap < (1LL << 32) - (1LL << 24), "experts * max_n must be below 2^32 - 2^24");
-  const long long units = (long long)a.E * a.cap * ceil_div_i(a.K / kSfBlock, 32);
-  const bool loose = !aligned_to(a.b_act, 16) || !aligned_to(a.sfb, 16);
-  PNV_CUDA(launch_pdl(loose ? quant_batched_kernel<kSrc, true> : quant_batched_kernel<kSrc, false>,
+  const int KB = a.K / kSfBlock;
+  // A warp per row where rows are long (64 K-blocks) and at most a sixteenth of its lanes would idle: the row's addresses
+  // and its lookup then serve many blocks.
+  const bool rows = KB >= 64 && 16 * (round_up_i(KB, 32) - KB) <= KB && aligned_to(a.b_act, 16) && aligned_to(a.sfb, 16);
+  const long long units = rows ? (long long)a.E * a.cap * ceil_div_i(KB, 32) : ((long long)a.E * a.cap * sf_k_atoms(a.K) + 7) / 8;
+  PNV_CUDA(launch_pdl(rows ? quant_batched_kernel<kSrc> : quant_quads_kernel<kSrc>,
                       dim3(grid_for(units, sm_count, kBatchedBlocks)), dim3(kThreads), live_rows_smem(a.E), s, pdl_enabled(), a));
   return PNV_OK;
 }

@@ -54,6 +54,37 @@ def test_quant_act_and_planned_scatter(ops, E, cap, K, counts, offset):
     assert np.array_equal(u8(b2)[written], ob2[written]) and np.array_equal(u8(sf2), osf2)
 
 
+LOOKUP_CASES = [
+    # E, cap, K: rows and quads - what a warp looks up at once, and where its range starts and ends inside a row
+    (3, 100003, 32),       # one quad a row, more than 32 rows to a warp
+    (8500, 37, 32),        # ... without prefix sums, most of them dead
+    (50, 331, 288),        # three quads a row, the last with one K-block
+    (5, 2, 2112),          # 17 quads a row, fewer rows than warps; K-blocks that leave the row form's lanes idle
+    (40, 90, 2080),        # the same with more
+    (40, 200, 2048),       # the row form, prefix in shared memory
+]
+
+
+@pytest.mark.parametrize("E,cap,K", LOOKUP_CASES)
+def test_every_row_is_found_once(ops, E, cap, K):
+    rng = np.random.default_rng(E * K)
+    cnt = (rng.integers(0, cap + 1, E) * (rng.random(E) < (0.2 if E > 1000 else 0.9))).astype(np.int32)
+    xb = make_acts(E, cap, K, seed=E + K)
+    g = rng.uniform(1.0, 40.0, E).astype(np.float32)
+    b, sf = ops.quant_act(bf16_tensor(xb), dev(g), dev(cnt), 128)
+    ob, valid, osf = orc.quant_act(xb, g, cnt)
+    assert np.array_equal(u8(b)[valid], ob[valid]) and np.array_equal(u8(sf), osf)
+    # the gated form and the gather against the plain one, on the GPU
+    x2 = bf16_tensor(np.concatenate([xb, xb[..., ::-1]], axis=-1))
+    y = ops.gated_act(x2, False)
+    vt = torch.from_numpy(valid).cuda()
+    got, want = ops.silu_mul_quant_act(x2, dev(g), dev(cnt), 128, False), ops.quant_act(y, dev(g), dev(cnt), 128)
+    assert torch.equal(got[0][vt], want[0][vt]) and torch.equal(got[1], want[1])
+    src = dev(np.arange(E * cap, dtype=np.int32))
+    got = ops.scatter_quant_act_planned(y.view(E * cap, K), src, src, None, dev(g), dev(cnt), cap)
+    assert torch.equal(got[0][vt], want[0][vt]) and torch.equal(got[1], want[1])
+
+
 @pytest.mark.parametrize("T,topk,E,cap", [(1, 1, 1, 1), (5, 7, 512, 3), (5, 7, 513, 3), (128, 8, 512, 40), (147, 7, 600, 9),
                                           (1500, 3, 512, 12), (1500, 3, 4096, 2), (341, 3, 8, 1000)])
 def test_plan_around_the_ranking_tables_limit(ops, T, topk, E, cap):
