@@ -466,11 +466,71 @@ __device__ __forceinline__ void warp_copy(const uint4* __restrict__ src, uint4* 
 }
 constexpr int kCopyBlocks = 3;      // blocks per SM of the kernels that copy rows (80 registers)
 
+// One word of scales: K-blocks 4 kt ... of a row in natural order (`words`: the row can be read by aligned words); blocks
+// past K become the benign byte.
+__device__ __forceinline__ uint32_t load_sf_word(const uint8_t* sf_src, int kt, int KB, bool words) {
+  if (words) return __ldg(reinterpret_cast<const uint32_t*>(sf_src) + kt);
+  uint32_t w = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) w |= (kt * 4 + i < KB ? (uint32_t)__ldg(sf_src + kt * 4 + i) : (uint32_t)kBenignSf) << (8 * i);
+  return w;
+}
+__device__ __forceinline__ void store_sf_word(uint8_t* dst, uint32_t w, bool dst4) {
+  if (dst4) {
+    *reinterpret_cast<uint32_t*>(dst) = w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dst[i] = (uint8_t)(w >> (8 * i));
+  }
+}
+
 // scatter_fp4_planned / scatter_fp4_wire: already quantized rows into the batched operands, one warp per live row.
 // Codes are copied 16 bytes per lane; the row's scales go from natural order into the swizzled layout four
 // K-blocks (one aligned word of both layouts) at a time.  Slots at or past counts[e] get the benign fill in their scales.
+// A warp looks up its next 32 rows at once, one per lane, and copies short rows two or four at a time: the search,
+// the source index and the row's first load are a chain of three memory latencies that long rows hide and short ones do not.
 // Bound: HBM (65536 rows of 7168: 250 MB in and out in 104 us; a plain fill of 256 MB takes 74).
-__global__ void __launch_bounds__(kThreads)
+struct Fp4Rows {
+  const uint8_t* q;
+  const uint8_t* q_sf;
+  uint8_t* b_act;
+  uint8_t* sfb;
+  long long q_pitch, sf_pitch;
+  int K, KB, cap, n_rt, n_kt;
+  bool words, dst4;
+};
+// Rows i0 ... i0 + kRows - 1 of the 32 looked up (slot, token and expert of row i in lane i; expert -1: none).
+template <int kRows, int kVecs>                // kVecs: 16-byte words of a row per lane
+__device__ __forceinline__ void copy_fp4_rows(const Fp4Rows& a, int i0, int my_e, unsigned my_slot, int my_tok, int lane) {
+  const int nv = a.K / 32;
+  uint4 x[kRows * kVecs];
+  uint32_t sf[kRows];
+#pragma unroll
+  for (int g = 0; g < kRows; ++g) {
+    const bool on = __shfl_sync(0xffffffffu, my_e, i0 + g) >= 0;
+    const long long t = __shfl_sync(0xffffffffu, my_tok, i0 + g);
+    const uint4* src = reinterpret_cast<const uint4*>(a.q + t * a.q_pitch);
+    if (on && lane < a.n_kt) sf[g] = load_sf_word(a.q_sf + t * a.sf_pitch, lane, a.KB, a.words);
+#pragma unroll
+    for (int c = 0; c < kVecs; ++c)
+      if (on && c * 32 + lane < nv) x[g * kVecs + c] = __ldg(src + c * 32 + lane);
+  }
+#pragma unroll
+  for (int g = 0; g < kRows; ++g) {
+    const int e = __shfl_sync(0xffffffffu, my_e, i0 + g);
+    const unsigned slot = __shfl_sync(0xffffffffu, my_slot, i0 + g);
+    if (e < 0) continue;
+    uint4* dst = reinterpret_cast<uint4*>(a.b_act + (long long)slot * (a.K / 2));
+    if (lane < a.n_kt)
+      store_sf_word(a.sfb + sf_offset(e, (int)(slot - (unsigned)e * (unsigned)a.cap), lane * 4, a.n_rt, a.n_kt), sf[g], a.dst4);
+#pragma unroll
+    for (int c = 0; c < kVecs; ++c)
+      if (c * 32 + lane < nv) dst[c * 32 + lane] = x[g * kVecs + c];
+  }
+}
+// kRows: rows a warp copies at a time, each of at most 32 * kVecs 16-byte words; 1: long rows, one after the other.
+template <int kRows, int kVecs>
+__global__ void __launch_bounds__(kThreads, kCopyBlocks)
 scatter_fp4_rows_kernel(const uint8_t* __restrict__ q, long long q_pitch, const uint8_t* __restrict__ q_sf,
                         long long sf_pitch, const int* __restrict__ src_tok, const int* __restrict__ counts, int K, int E,
                         int cap, uint8_t* __restrict__ b_act, uint8_t* __restrict__ sfb) {
@@ -478,30 +538,41 @@ scatter_fp4_rows_kernel(const uint8_t* __restrict__ q, long long q_pitch, const 
   pdl_wait();
   pdl_launch_dependents();
   const int KB = K / kSfBlock;
-  const int n_rt = sf_row_atoms(cap);
-  const int n_kt = sf_k_atoms(K);
+  const bool words = (KB % 4) == 0 && (sf_pitch % 4) == 0 && (reinterpret_cast<uintptr_t>(q_sf) % 4) == 0;
+  const Fp4Rows a{q, q_sf, b_act, sfb, q_pitch, sf_pitch, K, KB, cap, sf_row_atoms(cap), sf_k_atoms(K), words,
+                  (reinterpret_cast<uintptr_t>(sfb) % 4) == 0};
   const int lane = threadIdx.x & 31;
   LiveRows rows;
   rows.make(counts, E, cap, s_prefix);
   const unsigned nwarps = gridDim.x * kWarpsPerBlock;
-  const bool words = (KB % 4) == 0 && (sf_pitch % 4) == 0 && ((reinterpret_cast<uintptr_t>(q_sf) | reinterpret_cast<uintptr_t>(sfb)) % 4) == 0;
-  for (unsigned j = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); j < rows.total; j += nwarps) {
-    int e, r;
-    if (!rows.find(j, e, r)) continue;
-    const long long slot = (long long)e * cap + r;
-    const long long t = src_tok[slot];
-    const uint8_t* sf_src = q_sf + t * sf_pitch;
-    uint8_t* sf_row = sfb + sf_offset(e, r, 0, n_rt, n_kt);        // K-block kb of this row: + (kb >> 2) * 512 + (kb & 3)
-    if (words) {
-      for (int w = lane; w < KB / 4; w += 32)
-        *reinterpret_cast<uint32_t*>(sf_row + w * 512) = __ldg(reinterpret_cast<const uint32_t*>(sf_src) + w);
+  for (unsigned j0 = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); j0 < rows.total; j0 += 32u * nwarps) {
+    const unsigned long long j = j0 + (unsigned long long)lane * nwarps;  // this lane looks up the warp's row number `lane`
+    const bool there = j < rows.total;
+    int e, r, tok = 0;
+    rows.find_each(there ? (unsigned)j : j0, e, r);
+    if (!there) e = -1;
+    const unsigned slot = e < 0 ? 0u : (unsigned)e * (unsigned)cap + (unsigned)r;
+    if (e >= 0) tok = src_tok[slot];
+    const int n = (int)min(32u, (rows.total - j0 + nwarps - 1) / nwarps);
+    if constexpr (kRows > 1) {
+#pragma unroll 1
+      for (int i = 0; i < n; i += kRows) copy_fp4_rows<kRows, kVecs>(a, i, e, slot, tok, lane);
     } else {
-      for (int kb = lane; kb < n_kt * 4; kb += 32)      // (blocks past K keep the benign byte in the layout's slop)
-        sf_row[(kb >> 2) * 512 + (kb & 3)] = kb < KB ? __ldg(sf_src + kb) : (uint8_t)kBenignSf;
+#pragma unroll 1
+      for (int i = 0; i < n; ++i) {
+        const int ei = __shfl_sync(0xffffffffu, e, i);
+        const unsigned si = __shfl_sync(0xffffffffu, slot, i);
+        const long long t = __shfl_sync(0xffffffffu, tok, i);
+        if (ei < 0) continue;
+        uint8_t* sf_row = sfb + sf_offset(ei, (int)(si - (unsigned)ei * (unsigned)cap), 0, a.n_rt, a.n_kt);
+#pragma unroll 1
+        for (int kt = lane; kt < a.n_kt; kt += 32)
+          store_sf_word(sf_row + kt * 512, load_sf_word(q_sf + t * sf_pitch, kt, KB, words), a.dst4);
+        warp_copy(reinterpret_cast<const uint4*>(q + t * q_pitch), reinterpret_cast<uint4*>(b_act + (long long)si * (K / 2)), K / 32, lane);
+      }
     }
-    warp_copy(reinterpret_cast<const uint4*>(q + t * q_pitch), reinterpret_cast<uint4*>(b_act + slot * (K / 2)), K / 32, lane);
   }
-  benign_fill_dead<true>(counts, E, cap, n_rt, n_kt, sfb);
+  benign_fill_dead<true>(counts, E, cap, a.n_rt, a.n_kt, sfb);
 }
 
 // quant_rows: token-order rows -> row-major codes and natural-order scales, one shared global scale.
@@ -774,7 +845,10 @@ int scatter_fp4_rows(const uint8_t* q, long long q_pitch, const uint8_t* q_sf, l
   PNV_REQUIRE((long long)experts * cap < (1LL << 31), "E * cap must fit int32");
   PNV_REQUIRE((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(b_act) | (uintptr_t)q_pitch) % 16 == 0,
               "code rows must be 16-byte aligned");
-  PNV_CUDA(launch_pdl(scatter_fp4_rows_kernel, dim3(grid_for((long long)experts * cap, sm_count, kCopyBlocks)), dim3(kThreads),
+  const int nv = k / 32;
+  auto kernel = nv <= 32 ? scatter_fp4_rows_kernel<4, 1> : nv <= 64 ? scatter_fp4_rows_kernel<4, 2>
+              : nv <= 128 ? scatter_fp4_rows_kernel<2, 4> : scatter_fp4_rows_kernel<1, 8>;
+  PNV_CUDA(launch_pdl(kernel, dim3(grid_for((long long)experts * cap, sm_count, kCopyBlocks)), dim3(kThreads),
                       live_rows_smem(experts), s, pdl_enabled(), q, q_pitch, q_sf, sf_pitch, (const int*)src_tok,
                       (const int*)counts, k, experts, cap, b_act, sfb));
   return PNV_OK;
