@@ -132,6 +132,16 @@ scatter_quant_kernel(const __nv_bfloat16* __restrict__ a1, const long long* __re
   }
 }
 
+// One word of scales.
+__device__ __forceinline__ void store_sf_word(uint8_t* dst, uint32_t w, bool dst4) {
+  if (dst4) {
+    *reinterpret_cast<uint32_t*>(dst) = w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dst[i] = (uint8_t)(w >> (8 * i));
+  }
+}
+
 // Every byte of a scale buffer that no live row (r < counts[e]) writes becomes 0x38: whole 16-byte lines behind which
 // no row is live, single words of the others.  (K-block slop of a live row is part of the words that row writes.)  The
 // kernels that place rows do this themselves, each thread a share of the lines: as a memset in front of them it was a
@@ -155,14 +165,35 @@ __device__ __forceinline__ void benign_fill_dead(const int* __restrict__ counts,
     } else {
 #pragma unroll
       for (int g = 0; g < 4; ++g)
-        if (r0 + 32 * g >= cnt) {
-          if (sfb4) {
-            *reinterpret_cast<uint32_t*>(line + 4 * g) = w4;
-          } else {
+        if (r0 + 32 * g >= cnt) store_sf_word(line + 4 * g, w4, sfb4);
+    }
+  }
+}
+
+// The same for the kernel that copies rows: neighbouring atoms of a row atom per warp, up to eight where every warp has as
+// many to do, so that the divisions and the count serve eight stores a lane.  (2048 experts x 4 rows x 7168: 28 us with a
+// line per thread, 23 so.  The quantizers' small calls are a microsecond faster with a line per thread.)
+__device__ __forceinline__ void benign_fill_dead_atoms(const int* __restrict__ counts, int E, int cap, int n_rt, int n_kt,
+                                                       uint8_t* __restrict__ sfb) {
+  const uint32_t w4 = kBenignSf * 0x01010101u;
+  const bool sfb16 = (reinterpret_cast<uintptr_t>(sfb) & 15) == 0, sfb4 = (reinterpret_cast<uintptr_t>(sfb) & 3) == 0;
+  const unsigned nwarps = gridDim.x * kWarpsPerBlock, lane = threadIdx.x & 31;
+  const unsigned per_unit = min(8u, max(1u, (unsigned)E * n_rt * n_kt / nwarps));
+  const unsigned n_kc = ((unsigned)n_kt + per_unit - 1) / per_unit, units = (unsigned)E * n_rt * n_kc;
+  for (unsigned u = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < units; u += nwarps) {
+    const unsigned row_atom = u / n_kc, kt0 = (u - row_atom * n_kc) * per_unit, e = row_atom / (unsigned)n_rt;
+    const int base = (int)(row_atom - e * (unsigned)n_rt) * 128, r0 = base + (int)lane, cnt = min(counts[e], cap);
+    if (cnt - base >= 128) continue;                      // (every row of these atoms is live)
+    const unsigned n = min(per_unit, (unsigned)n_kt - kt0);
+    uint8_t* line = sfb + ((long long)row_atom * n_kt + kt0) * 512 + lane * 16;
+    if (r0 >= cnt && sfb16) {
+      for (unsigned i = 0; i < n; ++i) *reinterpret_cast<uint4*>(line + i * 512) = make_uint4(w4, w4, w4, w4);
+    } else {
+      for (unsigned i = 0; i < n; ++i) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) line[4 * g + i] = (uint8_t)kBenignSf;
-          }
-        }
+        for (int g = 0; g < 4; ++g)
+          if (r0 + 32 * g >= cnt) store_sf_word(line + i * 512 + 4 * g, w4, sfb4);
+      }
     }
   }
 }
@@ -195,31 +226,47 @@ struct LiveRows {
       total = __shfl_sync(0xffffffffu, v, 31);
       return;
     }
+    // Every thread takes a run of counts (one up to 256 experts; otherwise they go through shared memory by independent
+    // loads, and a run of odd length has no bank conflicts), the runs' sums are scanned over the block, and every thread
+    // turns its run into prefix sums in place.  (256 counts at a time, a global load and two barriers each, took 7 us for
+    // 4096 experts.)
     __shared__ unsigned s_warp[kWarpsPerBlock];
-    unsigned carry = 0;
-    for (int e0 = 0; e0 < E; e0 += kThreads) {
-      const int e = e0 + (int)threadIdx.x;
-      unsigned v = e < E ? (unsigned)max(0, min(counts[e], cap)) : 0u;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned u = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += u;
-      }
-      if (lane == 31) s_warp[warp] = v;
+    auto count = [&](int e) { return (unsigned)max(0, min(counts[e], cap)); };
+    const int run = ((E + kThreads - 1) / kThreads) | 1, lo = (int)threadIdx.x * run, hi = min(E, lo + run);
+    unsigned sum = 0;
+    if (run == 1) {
+      if (lo < E) sum = count(lo);
+    } else {
+#pragma unroll 4
+      for (int e = threadIdx.x; e < E; e += kThreads) smem[e + 1] = count(e);
       __syncthreads();
-      unsigned before = carry, sum = 0;
+      for (int e = lo; e < hi; ++e) sum += smem[e + 1];
+    }
+    unsigned v = sum;
 #pragma unroll
-      for (int i = 0; i < kWarpsPerBlock; ++i) {
-        if (i < warp) before += s_warp[i];
-        sum += s_warp[i];
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned u = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += u;
+    }
+    if (lane == 31) s_warp[warp] = v;
+    __syncthreads();
+    unsigned before = v - sum, all = 0;
+#pragma unroll
+    for (int i = 0; i < kWarpsPerBlock; ++i) {
+      if (i < warp) before += s_warp[i];
+      all += s_warp[i];
+    }
+    if (run == 1) {
+      if (lo < E) smem[lo + 1] = before + sum;
+    } else {
+      for (int e = lo; e < hi; ++e) {
+        before += smem[e + 1];
+        smem[e + 1] = before;
       }
-      if (e < E) smem[e + 1] = before + v;
-      carry += sum;
-      __syncthreads();
     }
     if (threadIdx.x == 0) smem[0] = 0;
     __syncthreads();
-    total = carry;
+    total = all;
   }
   // row number j < total -> expert and row of the expert; false for a dead slot (only without prefix sums)
   __device__ __forceinline__ bool find(unsigned j, int& e, int& r) const {
@@ -282,6 +329,7 @@ struct RowsArgs {
   uint8_t* sfb;
   GatedAct act;
   int gscale_per_expert, E, cap, K, interleaved;
+  int filled;            // the scale buffer already holds the benign byte everywhere
 };
 
 // Blocks per SM: four hold 64 registers a thread; five or six spill (6 to 17 % slower with the activation), three with the
@@ -351,7 +399,7 @@ quant_batched_kernel(const RowsArgs a) {
       finish_blocks(b, kb0, KB, gs, dst, sf_row, lane);
     }
   }
-  benign_fill_dead<false>(a.counts, a.E, a.cap, n_rt, n_kt, a.sfb);
+  if (!a.filled) benign_fill_dead<false>(a.counts, a.E, a.cap, n_rt, n_kt, a.sfb);
 }
 
 // The same for short rows, rows that leave many lanes of a warp's last 32 K-blocks idle, and destinations that are less
@@ -449,7 +497,7 @@ quant_quads_kernel(const RowsArgs a) {
       if (kt >= n_kt) { kt -= n_kt; ++b; }
     }
   }
-  benign_fill_dead<true>(a.counts, a.E, a.cap, n_rt, n_kt, a.sfb);
+  if (!a.filled) benign_fill_dead<true>(a.counts, a.E, a.cap, n_rt, n_kt, a.sfb);
 }
 
 // n 16-byte words by one warp, eight of them per lane in flight.
@@ -475,15 +523,6 @@ __device__ __forceinline__ uint32_t load_sf_word(const uint8_t* sf_src, int kt, 
   for (int i = 0; i < 4; ++i) w |= (kt * 4 + i < KB ? (uint32_t)__ldg(sf_src + kt * 4 + i) : (uint32_t)kBenignSf) << (8 * i);
   return w;
 }
-__device__ __forceinline__ void store_sf_word(uint8_t* dst, uint32_t w, bool dst4) {
-  if (dst4) {
-    *reinterpret_cast<uint32_t*>(dst) = w;
-  } else {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) dst[i] = (uint8_t)(w >> (8 * i));
-  }
-}
-
 // scatter_fp4_planned / scatter_fp4_wire: already quantized rows into the batched operands, one warp per live row.
 // Codes are copied 16 bytes per lane; the row's scales go from natural order into the swizzled layout four
 // K-blocks (one aligned word of both layouts) at a time.  Slots at or past counts[e] get the benign fill in their scales.
@@ -533,7 +572,7 @@ template <int kRows, int kVecs>
 __global__ void __launch_bounds__(kThreads, kCopyBlocks)
 scatter_fp4_rows_kernel(const uint8_t* __restrict__ q, long long q_pitch, const uint8_t* __restrict__ q_sf,
                         long long sf_pitch, const int* __restrict__ src_tok, const int* __restrict__ counts, int K, int E,
-                        int cap, uint8_t* __restrict__ b_act, uint8_t* __restrict__ sfb) {
+                        int cap, uint8_t* __restrict__ b_act, uint8_t* __restrict__ sfb, int filled) {
   extern __shared__ unsigned s_prefix[];
   pdl_wait();
   pdl_launch_dependents();
@@ -572,7 +611,7 @@ scatter_fp4_rows_kernel(const uint8_t* __restrict__ q, long long q_pitch, const 
       }
     }
   }
-  benign_fill_dead<true>(counts, E, cap, a.n_rt, a.n_kt, sfb);
+  if (!filled) benign_fill_dead_atoms(counts, E, cap, a.n_rt, a.n_kt, sfb);
 }
 
 // quant_rows: token-order rows -> row-major codes and natural-order scales, one shared global scale.
@@ -708,20 +747,41 @@ int check_common(const void* x, const float* gscale, const int32_t* counts, int 
   return PNV_OK;
 }
 
+// The planned scatters' fill.  Rows between the capacity and the end of its last 128-row atom are dead whatever the counts
+// say.  Where they are many - thousands of experts of a few rows - the whole scale buffer is filled by a memset first, which
+// writes faster than the row kernels' own fill; otherwise the row kernels do it and can start while their predecessor
+// drains.  The lines, measured: rows copied for 2048 experts x 16 x 7168 (49 MiB surely dead) 58 us with a memset, 62
+// without, below that the memset loses; rows quantized for 2048 experts 92 us with, 85 without, for 9000 x 4 x 7168
+// (238 MiB) 137 with, 160 without.
+constexpr long long kMemsetFillCopy = 40LL << 20, kMemsetFillQuant = 96LL << 20;
+int fill_ahead(uint8_t* sfb, int E, int cap, int K, long long least, cudaStream_t s, int& filled) {
+  const long long surely_dead = (long long)E * ((long long)sf_row_atoms(cap) * 128 - cap) * sf_k_atoms(K) * 4;
+  filled = surely_dead >= least ? 1 : 0;
+  if (filled) PNV_CUDA(cudaMemsetAsync(sfb, kBenignSf, (size_t)sf_numel(cap, K, E), s));
+  return PNV_OK;
+}
+
 // One launch of the shared kernel: at most a wave of warps, one per 32 K-blocks of a row of the capacity (or eight quads).
 template <int kSrc>
-int launch_batched(const RowsArgs& a, int sm_count, cudaStream_t s) {
+int launch_batched(RowsArgs a, int sm_count, cudaStream_t s) {
   if (int rc = check_alignment(a.x, a.b_act, kSrc == kGather ? 16 : 8, a.sfb)) return rc;
   if (kSrc == kGather) PNV_REQUIRE((long long)a.E * a.cap < (1LL << 31), "E * cap must fit int32");
   // (a grid stride short of 2^32, so that a warp's next row number cannot wrap around)
   PNV_REQUIRE((long long)a.E * a.cap < (1LL << 32) - (1LL << 24), "experts * max_n must be below 2^32 - 2^24");
+  if (kSrc == kGather)
+    if (int rc = fill_ahead(a.sfb, a.E, a.cap, a.K, kMemsetFillQuant, s, a.filled)) return rc;
   const int KB = a.K / kSfBlock;
   // A warp per row where rows are long (64 K-blocks) and at most a sixteenth of its lanes would idle: the row's addresses
-  // and its lookup then serve many blocks.
-  const bool rows = KB >= 64 && 16 * (round_up_i(KB, 32) - KB) <= KB && aligned_to(a.b_act, 16) && aligned_to(a.sfb, 16);
-  const long long units = rows ? (long long)a.E * a.cap * ceil_div_i(KB, 32) : ((long long)a.E * a.cap * sf_k_atoms(a.K) + 7) / 8;
+  // and its lookup then serve many blocks.  Also where the whole capacity is no more than one step for each warp of a wave:
+  // idle lanes then cost nothing, and the row form starts sooner (the grouped linear layer of 5 experts x 1 row x 4608: 13.0
+  // us against 13.3).
+  const long long steps = (long long)a.E * a.cap * ceil_div_i(KB, 32);
+  const long long wave = (long long)(sm_count > 0 ? sm_count : 148) * kBatchedBlocks * kWarpsPerBlock;
+  const bool rows = aligned_to(a.b_act, 16) && aligned_to(a.sfb, 16) &&
+                    (steps <= wave || (KB >= 64 && 16 * (round_up_i(KB, 32) - KB) <= KB));
+  const long long units = rows ? steps : ((long long)a.E * a.cap * sf_k_atoms(a.K) + 7) / 8;
   PNV_CUDA(launch_pdl(rows ? quant_batched_kernel<kSrc> : quant_quads_kernel<kSrc>,
-                      dim3(grid_for(units, sm_count, kBatchedBlocks)), dim3(kThreads), live_rows_smem(a.E), s, pdl_enabled(), a));
+                      dim3(grid_for(units, sm_count, kBatchedBlocks)), dim3(kThreads), live_rows_smem(a.E), s, pdl_enabled() && !a.filled, a));
   return PNV_OK;
 }
 
@@ -750,7 +810,7 @@ extern "C" int pnv_quant_act(const void* x, const float* gscale, int gscale_per_
                              uint8_t* sfb, int sm_count, pnv_stream_t stream) {
   if (int rc = check_common(x, gscale, counts, experts, max_n, k, b_act, sfb, "K")) return rc;
   RowsArgs a{(const __nv_bfloat16*)x, nullptr, nullptr, nullptr, gscale, (const int*)counts, b_act, sfb, GatedAct{},
-             gscale_per_expert, experts, max_n, k, 0};
+             gscale_per_expert, experts, max_n, k, 0, 0};
   return launch_batched<kPlain>(a, sm_count, (cudaStream_t)stream);
 }
 
@@ -764,7 +824,7 @@ extern "C" int pnv_silu_mul_quant_act(const void* x2, const float* gscale, int g
   if (int rc = check_common(x2, gscale, counts, experts, max_n, n, b_act, sfb, "intermediate width N"))
     return rc;
   RowsArgs a{(const __nv_bfloat16*)x2, nullptr, nullptr, nullptr, gscale, (const int*)counts, b_act, sfb, act,
-             gscale_per_expert, experts, max_n, n, interleaved ? 1 : 0};
+             gscale_per_expert, experts, max_n, n, interleaved ? 1 : 0, 0};
   return launch_batched<kGated>(a, sm_count, (cudaStream_t)stream);
 }
 
@@ -818,7 +878,7 @@ extern "C" int pnv_scatter_quant_act_planned(const void* a1, const int32_t* src_
   PNV_REQUIRE(src_tok && src_route, "null pointer argument");
   if (int rc = check_common(a1, gscale, counts, experts, cap, k, b_act, sfb, "K")) return rc;
   RowsArgs a{(const __nv_bfloat16*)a1, (const int*)src_tok, (const int*)src_route, topk_weights, gscale, (const int*)counts,
-             b_act, sfb, GatedAct{}, gscale_per_expert, experts, cap, k, 0};
+             b_act, sfb, GatedAct{}, gscale_per_expert, experts, cap, k, 0, 0};
   return launch_batched<kGather>(a, sm_count, (cudaStream_t)stream);
 }
 
@@ -845,12 +905,14 @@ int scatter_fp4_rows(const uint8_t* q, long long q_pitch, const uint8_t* q_sf, l
   PNV_REQUIRE((long long)experts * cap < (1LL << 31), "E * cap must fit int32");
   PNV_REQUIRE((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(b_act) | (uintptr_t)q_pitch) % 16 == 0,
               "code rows must be 16-byte aligned");
+  int filled = 0;
+  if (int rc = fill_ahead(sfb, experts, cap, k, kMemsetFillCopy, s, filled)) return rc;
   const int nv = k / 32;
   auto kernel = nv <= 32 ? scatter_fp4_rows_kernel<4, 1> : nv <= 64 ? scatter_fp4_rows_kernel<4, 2>
               : nv <= 128 ? scatter_fp4_rows_kernel<2, 4> : scatter_fp4_rows_kernel<1, 8>;
   PNV_CUDA(launch_pdl(kernel, dim3(grid_for((long long)experts * cap, sm_count, kCopyBlocks)), dim3(kThreads),
-                      live_rows_smem(experts), s, pdl_enabled(), q, q_pitch, q_sf, sf_pitch, (const int*)src_tok,
-                      (const int*)counts, k, experts, cap, b_act, sfb));
+                      live_rows_smem(experts), s, pdl_enabled() && !filled, q, q_pitch, q_sf, sf_pitch, (const int*)src_tok,
+                      (const int*)counts, k, experts, cap, b_act, sfb, filled));
   return PNV_OK;
 }
 }  // namespace

@@ -85,6 +85,23 @@ def test_every_row_is_found_once(ops, E, cap, K):
     assert torch.equal(got[0][vt], want[0][vt]) and torch.equal(got[1], want[1])
 
 
+@pytest.mark.parametrize("E,cap,K", [(4090, 1, 6272), (200, 130, 1056), (160, 70, 2080)])      # filled ahead (97 MiB surely dead); by the kernel
+def test_planned_scatters_fill_every_dead_scale(ops, E, cap, K):
+    rng = np.random.default_rng(E)
+    cnt = rng.integers(0, cap + 1, E).astype(np.int32)
+    T = 40
+    xb = make_acts(1, T, K, seed=K)[0]
+    src = rng.integers(0, T, E * cap).astype(np.int32)
+    g = np.array([3.0], np.float32)
+    live = np.arange(cap)[None, :] < cnt[:, None]
+    dest = np.where(live.reshape(-1), np.arange(E * cap), E * cap).astype(np.int64)
+    q, q_sf = ops.quant_rows(bf16_tensor(xb), dev(g))
+    ob, written, osf = orc.scatter_quant_act(xb, src, dest, None, g, E, cap)
+    for b, sf in (ops.scatter_quant_act_planned(bf16_tensor(xb), dev(src), dev(src), None, dev(g), dev(cnt), cap),
+                  ops.scatter_fp4_planned(q, q_sf, dev(src), dev(cnt), cap)):
+        assert np.array_equal(u8(sf), osf) and np.array_equal(u8(b)[written], ob[written])
+
+
 @pytest.mark.parametrize("T,topk,E,cap", [(1, 1, 1, 1), (5, 7, 512, 3), (5, 7, 513, 3), (128, 8, 512, 40), (147, 7, 600, 9),
                                           (1500, 3, 512, 12), (1500, 3, 4096, 2), (341, 3, 8, 1000)])
 def test_plan_around_the_ranking_tables_limit(ops, T, topk, E, cap):
