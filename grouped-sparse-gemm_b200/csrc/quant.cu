@@ -649,27 +649,27 @@ quant_rows_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__
   }
 }
 
+// The activation alone, 16 features (32 bytes of gate, up and result) per thread.  Bound: HBM (131072 rows of 2 x 2048).
 __global__ void __launch_bounds__(kThreads)
 gated_act_kernel(const __nv_bfloat16* __restrict__ x2, long long rows, int N, int interleaved,
                  GatedAct act, __nv_bfloat16* __restrict__ y) {
-  const int per_row = N / 8;
+  const int per_row = N / 16;
   const long long total = rows * per_row;
+  const bool wide = (reinterpret_cast<uintptr_t>(x2) & 31) == 0;
   for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
     const long long row = idx / per_row;
-    const int k0 = (int)(idx - row * per_row) * 8;
+    const int k0 = (int)(idx - row * per_row) * 16;
     const __nv_bfloat16* base = x2 + row * (2LL * N);
     const int gate_off = interleaved ? (k0 / 32) * 64 + (k0 % 32) : k0;
     const int up_off = interleaved ? gate_off + 32 : N + k0;
-    uint4 gv = __ldg(reinterpret_cast<const uint4*>(base + gate_off));
-    uint4 uv = __ldg(reinterpret_cast<const uint4*>(base + up_off));
-    float ga[8], ua[8];
-    unpack8(gv, ga);
-    unpack8(uv, ua);
-    __nv_bfloat16 o[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] = __float2bfloat16_rn(gated_act(ga[i], ua[i], act));
-    *reinterpret_cast<uint4*>(y + row * N + k0) = *reinterpret_cast<const uint4*>(o);
+    uint32_t g[8], u[8], o[8];
+    load32(reinterpret_cast<const uint8_t*>(base + gate_off), wide, g);
+    load32(reinterpret_cast<const uint8_t*>(base + up_off), wide, u);
+    gated_act16(g, u, act, o);
+    uint4* dst = reinterpret_cast<uint4*>(y + row * N + k0);
+    dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+    dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
   }
 }
 
@@ -861,7 +861,7 @@ extern "C" int pnv_gated_act(const void* x2, int64_t rows, int n, int interleave
   PNV_REQUIRE(n > 0 && n % kSfBlock == 0, "intermediate width N must be a multiple of %d, got %d", kSfBlock, n);
   if (rows <= 0) return PNV_OK;
   PNV_REQUIRE(aligned_to(x2, 16) && aligned_to(y, 16), "gated_act buffers must be 16-byte aligned");
-  long long total = rows * (n / 8);
+  long long total = rows * (n / 16);
   long long blocks = (total + kThreads - 1) / kThreads;
   if (blocks > 148LL * 32) blocks = 148LL * 32;
   gated_act_kernel<<<(unsigned)blocks, kThreads, 0, (cudaStream_t)stream>>>(

@@ -73,3 +73,13 @@ def test_planned_scatters(lib, K, sf_off):
         lib.check(call(b.data_ptr(), s.data_ptr()))
         assert same_rows(b, want[0], K) and torch.equal(s, want[1])
         assert untouched(fs, sf_off, n_sf)
+
+
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_gated_act_on_a_source_that_is_16_byte_aligned(interleaved):
+    ops = torch.ops.paired_nvfp4
+    x2 = bf16_tensor(make_acts(1, 37, 2 * 96, 3))[0]
+    flat = torch.empty(8 + x2.numel(), dtype=torch.bfloat16, device="cuda")
+    flat[8:] = x2.view(-1)
+    for act in (("silu", 1.0, -1.0), ("situ", 1.702, 1.0)):
+        assert torch.equal(ops.gated_act(flat[8:].view(37, 192), interleaved, *act), ops.gated_act(x2, interleaved, *act))
