@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from oracle import paired_nvfp4_oracle as orc
-from helpers import bf16_tensor, u8, dev, make_acts, make_weights
+from helpers import bf16_tensor, u8, dev, make_acts, make_weights, splits_k
 
 pytestmark = pytest.mark.gpu
 
@@ -147,7 +147,9 @@ ROW_MAP_CASES = [
     (3, 384, 768, 200, [200, 0, 77], (0, 1, 3, 5, 8)),       # wide kernels, single CTA and pairs, odd tile count
     (2, 250, 512, 300, [300, 150], (1, 2)),                  # 256-token tiles (two chunks per group); M tail
     (4, 768, 512, 330, [300, 257, 320, 64], (1,)),           # narrow tail tiles against two M units (three units: odd)
-    (4, 512, 2048, 16, [16, 0, 3, 9], (7,)),                 # narrow kernel, K split across CTAs
+    (4, 512, 2048, 16, [16, 0, 3, 9], (7,)),                 # narrow kernel, whole tiles
+    (4, 512, 4096, 16, [16, 0, 3, 9], (7,)),                 # narrow kernel, K split across CTAs
+    (3, 328, 3616, 32, [0, 32, 5], (7,)),                    # ... with a short last stage, M tail
     (2, 202, 1024, 32, [32, 20], (7,)),                      # narrow kernel, scalar store path (M % 8 != 0)
 ]
 
@@ -157,6 +159,7 @@ def test_group_mm_rows_permutes_the_output(pnk, E, M, K, max_n, counts, cids):
     """group_mm_rows == group_mm followed by a row permutation: kept rows land where the map says, bit for bit;
     rows mapped to -1 and rows no token maps to keep the caller's bytes."""
     ops = torch.ops.paired_nvfp4
+    assert splits_k(E, M, K, max_n, counts) == (K > 3072)
     packed, sf, _ = make_weights(E, M, K, 31)
     x = make_acts(E, max_n, K, 32)
     cnt = np.asarray(counts, np.int32)
@@ -193,8 +196,11 @@ def test_group_mm_rows_permutes_the_output(pnk, E, M, K, max_n, counts, cids):
 SPLIT_CASES = [
     # E, M, K, max_n, counts: decode-sized problems, where the K stages of all tiles are dealt evenly to the SMs
     (2, 256, 4096, 16, [16, 5]),                  # 4 tiles x 8 stages over 32 CTAs: every CTA gets one stage of a tile
-    (8, 512, 2048, 8, [0, 0, 0, 7, 0, 0, 0, 0]),  # one active expert: most CTAs get an empty range
-    (1, 128, 2176, 32, [32]),                     # K = 4 stages + a short tail stage that is a unit of its own
+    (8, 512, 3584, 8, [0, 0, 0, 7, 0, 0, 0, 0]),  # one active expert: most CTAs get an empty range
+    (1, 128, 3616, 32, [32]),                     # 7 stages + one K-block that is a unit of its own: one live issuer
+    (1, 256, 3840, 32, [17]),                     # ... two K-blocks: two live issuers
+    (2, 384, 4224, 16, [16, 2]),                  # 8 stages + a short one, three M tiles of two experts
+    (5, 1024, 7264, 32, [32, 0, 9, 1, 0]),        # ranges that end inside tiles, the last stage 96 deep
     (3, 384, 14336, 16, [16, 1, 9]),              # long K, tiles cut at arbitrary stages
     (8, 1024, 7168, 1, [0, 0, 0, 1, 0, 0, 0, 0]),   # one token on one expert (an expert-parallel decode rank)
 ]
@@ -205,6 +211,7 @@ def test_split_k_matches_oracle_and_unsplit(pnk, E, M, K, max_n, counts):
     """Through the operators the split is on (they keep a workspace per stream); through the C ABI with no
     workspace it is off.  Both must meet the bar; twice in a row, to show the counters return to zero."""
     from paired_nvfp4_kernels import _cabi
+    assert splits_k(E, M, K, max_n, counts), "the case no longer takes the path it is here for"
     ops = torch.ops.paired_nvfp4
     got_a, want, valid = run_case(pnk, E, M, K, max_n, counts, 7, seed=31)
     got_b, _, _ = run_case(pnk, E, M, K, max_n, counts, 7, seed=31)

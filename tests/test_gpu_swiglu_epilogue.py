@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from oracle import paired_nvfp4_oracle as orc
-from helpers import bf16_tensor, bf16_bits, u8, dev, make_acts
+from helpers import bf16_tensor, u8, dev, make_acts, splits_k
 
 pytestmark = pytest.mark.gpu
 
@@ -43,6 +43,8 @@ CASES = [
     (128, 1280, 6, 330, [257, 320, 330, 64, 321, 289]),   # narrow tail tiles (two M units per item) over one M unit
     (512, 256, 4, 580, [576, 300, 577, 290]),             # ... over four M units, a one-stage K loop
     (128, 3072, 3, 330, [257, 320, 64]),                  # ... with 512-K stages
+    (128, 3616, 8, 16, [0, 0, 9, 0, 0, 0, 0, 16]),        # decode on few active experts: K split across CTAs, short last stage
+    (320, 7168, 4, 32, [32, 0, 1, 17]),                   # ... ranges that end inside tiles
 ]
 
 
@@ -50,6 +52,7 @@ CASES = [
 @pytest.mark.parametrize("act,beta,lbeta", [("silu", 1.0, -1.0), ("situ", 1.702, 1.0), ("situ", 2.0, -1.0)])
 def test_fused_equals_unfused_bytes(pnk, N, K, E, max_n, counts, act, beta, lbeta):
     ops = torch.ops.paired_nvfp4
+    assert splits_k(E, 2 * N, K, max_n, counts) == (max_n <= 32 and K > 3072)
     o = build(N, K, E, max_n, counts, seed=N + K)
     g2 = dev(np.linspace(3.0, 40.0, E).astype(np.float32))
     valid = np.arange(max_n)[None, :] < o["counts"][:, None]
