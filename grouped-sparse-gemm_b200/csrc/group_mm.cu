@@ -63,8 +63,7 @@ enum Status : int {
 
 template <int TILE_N, int STAGE_K, int ISSUERS>
 struct Cfg {
-  static_assert(TILE_N == 16 || TILE_N == 32 || TILE_N == 64 || TILE_N == 128 || TILE_N == 256,
-                "tile widths: 16 and 32 (single token tile only), 64, 128, 256");
+  static_assert(TILE_N == 16 || TILE_N == 32, "tile widths: 16 and 32 (a single token tile per expert)");
   static_assert(ISSUERS == 1 || ISSUERS == 2 || ISSUERS == 4, "MMA issuer warps: 1, 2 or 4");
   static constexpr int kThreads = (6 + ISSUERS) * 32;
   static constexpr int kFirstEpilogueWarp = 2 + ISSUERS;
@@ -79,13 +78,11 @@ struct Cfg {
   static constexpr int kEAtoms = STAGE_K / 256;
   static constexpr int kEBytes = 2048 * kEAtoms;
   static constexpr int kSfaBytes = 512 * kAtoms;
-  static constexpr int kSfbRowAtoms = TILE_N > 128 ? 2 : 1;
-  static constexpr int kSfbBytes = kSfaBytes * kSfbRowAtoms;
+  static constexpr int kSfbBytes = kSfaBytes;
   static constexpr int kStageBytes = kABytes + kBBytes + kEBytes + kSfaBytes + kSfbBytes;
   static constexpr int kFixedBytes = 1024 + kOutStageBytes + 256 + 6 * kMaxExperts;
   static constexpr int kStages = (kSmemLimit - kFixedBytes) / kStageBytes;
-  static constexpr int kAccStages = TILE_N == 256 ? 1 : 2;
-  static constexpr int kSfbColsPerAtom = 4 * kSfbRowAtoms;
+  static constexpr int kAccStages = 2;
   static constexpr int kAtomsPerIssuer = kAtoms / ISSUERS;          // K-blocks of a stage per issuer
   static constexpr int kEAtomsPerIssuer = kAtomsPerIssuer >= 2 ? kAtomsPerIssuer / 2 : 1;
   static constexpr int kEColsPerIssuer = 4 * kEAtomsPerIssuer;      // private metadata columns
@@ -99,7 +96,7 @@ struct Cfg {
   static_assert(kStages >= 2, "not enough shared memory for a pipeline");
   static_assert(kAccStages * ISSUERS * TILE_N <= kColE, "accumulators overlap the metadata columns");
   static_assert(kColE + kEColsPerIssuer * ISSUERS <= kColSfa && kColSfa + 4 * kAtoms <= kColSfb &&
-                kColSfb + kSfbColsPerAtom * kAtoms <= kTmemCols, "tensor-memory column map overflows");
+                kColSfb + 4 * kAtoms <= kTmemCols, "tensor-memory column map overflows");
 };
 
 struct Params {
@@ -279,7 +276,6 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 
   UnitWalk walk;
   walk.init(s_active, n_active, p.n_mt, p.k_stages, p.split_counters != nullptr);
-  constexpr int n0 = 0;      // (a single token tile per expert)
   unsigned tile;
   int mt, ks0, ks1, slot;
 
@@ -305,11 +301,11 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           ptx::mbar_arrive_expect_tx(full_bar + stage, C::kABytes + (p.b_4d ? C::kBBoxes : b_boxes) * C::kBBoxBytes);
           ptx::tma_load_3d(st + C::kOffA, &map_a, full_bar + stage, ks * C::kARowBytes, mt * kTileM, e);
           if (p.b_4d) {
-            ptx::tma_load_4d(st + C::kOffB, &map_b, full_bar + stage, 0, n0, ks * C::kBBoxes, e);
+            ptx::tma_load_4d(st + C::kOffB, &map_b, full_bar + stage, 0, 0, ks * C::kBBoxes, e);
           } else {
             for (int b = 0; b < b_boxes; ++b)
               ptx::tma_load_3d(st + C::kOffB + b * C::kBBoxBytes, &map_b, full_bar + stage,
-                               ks * (STAGE_K / 2) + b * 128, n0, e);
+                               ks * (STAGE_K / 2) + b * 128, 0, e);
           }
         }
         __syncwarp();
@@ -331,8 +327,7 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const int e = walk.e;
       const uint8_t* e_base = p.e_meta + (((long long)e * p.e_k_atoms) * p.e_m_atoms + mt) * 2048;
       const uint8_t* sfa_base = p.sfa + (((long long)e * p.n_mt + mt) * p.n_kt) * 512;
-      const uint8_t* sfb_base = p.sfb + (((long long)e * p.sfb_rt + (n0 >> 7)) * p.n_kt) * 512;
-      const int sfb_row_atoms = TILE_N > 128 ? min(2, p.sfb_rt - (n0 >> 7)) : 1;
+      const uint8_t* sfb_base = p.sfb + ((long long)e * p.sfb_rt * p.n_kt) * 512;
 #pragma unroll 1
       for (int ks = ks0; ks < ks1; ++ks) {
         if (!ptx::mbar_wait_warp(empty_bar + stage, phase ^ 1)) {
@@ -345,14 +340,12 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const int e_atoms = (k_atoms + 1) / 2;
         const uint32_t sf_bytes = 512u * k_atoms;
         if (ptx::elect_one()) {
-          ptx::mbar_arrive_expect_tx(full_bar + stage, e_atoms * 2048 + sf_bytes * (1 + sfb_row_atoms));
+          ptx::mbar_arrive_expect_tx(full_bar + stage, e_atoms * 2048 + 2 * sf_bytes);
           for (int ea = 0; ea < e_atoms; ++ea)
             ptx::bulk_load(st + C::kOffE + ea * 2048,
                            e_base + (long long)(ks * C::kEAtoms + ea) * p.e_m_atoms * 2048, 2048, full_bar + stage);
           ptx::bulk_load(st + C::kOffSfa, sfa_base + (long long)ks * C::kAtoms * 512, sf_bytes, full_bar + stage);
-          for (int ra = 0; ra < sfb_row_atoms; ++ra)
-            ptx::bulk_load(st + C::kOffSfb + ra * C::kSfaBytes,
-                           sfb_base + ((long long)ra * p.n_kt + ks * C::kAtoms) * 512, sf_bytes, full_bar + stage);
+          ptx::bulk_load(st + C::kOffSfb, sfb_base + (long long)ks * C::kAtoms * 512, sf_bytes, full_bar + stage);
         }
         __syncwarp();
         if (++stage == p.stages) { stage = 0; phase ^= 1; }
@@ -409,11 +402,8 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             if (ka < k_atoms) {
               ptx::tc_cp_32x128b_warpx4(tmem_base + kColSfa + ka * 4,
                                         ptx::smem_desc(st + C::kOffSfa + ka * 512, 128, 0, 0));
-#pragma unroll
-              for (int ra = 0; ra < C::kSfbRowAtoms; ++ra)
-                ptx::tc_cp_32x128b_warpx4(
-                    tmem_base + kColSfb + ka * C::kSfbColsPerAtom + ra * 4,
-                    ptx::smem_desc(st + C::kOffSfb + ra * C::kSfaBytes + ka * 512, 128, 0, 0));
+              ptx::tc_cp_32x128b_warpx4(tmem_base + kColSfb + ka * 4,
+                                        ptx::smem_desc(st + C::kOffSfb + ka * 512, 128, 0, 0));
             }
           }
 #pragma unroll
@@ -427,7 +417,7 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
               const uint32_t e_tmem = e_cols + (kPer >= 2 ? i * 2 : (ka & 1) * 2);
               // the first MMA of a unit overwrites this issuer's partial accumulator
               ptx::tc_mma_sp_nvf4(d_tmem, a_desc, b_desc, idesc, ((ks - ks0) | i) != 0 ? 1u : 0u,
-                                  tmem_base + kColSfa + ka * 4, sfb_col + ka * C::kSfbColsPerAtom, e_tmem);
+                                  tmem_base + kColSfa + ka * 4, sfb_col + ka * 4, e_tmem);
             }
           }
           ptx::tc_commit(empty_bar + stage);     // stage reusable once every issuer's MMAs and copies retire
@@ -500,7 +490,7 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       const bool partial = ks0 > 0 || ks1 < p.k_stages;
 #pragma unroll 1
       for (int c0 = 0; c0 < TILE_N; c0 += 32) {
-        if (n0 + c0 >= cnt) break;             // uniform over the four epilogue warps
+        if (c0 >= cnt) break;             // uniform over the four epilogue warps
         uint32_t r[32];
         const uint32_t lane_base = tmem_base + ((uint32_t)(sub * 32) << 16) + c0;
         ptx::tc_ld_32x32(lane_base + (acc * ISSUERS) * TILE_N, r);
@@ -563,7 +553,7 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           epilogue_bar_sync();
           const int blk = (ep_tid >> 5) & 1, half = lane >> 4;
           const int t = (lane & 15) + 16 * (ep_tid >> 6);      // this lane's token column
-          const int n = n0 + c0 + t;
+          const int n = c0 + t;
           if (16 * (ep_tid >> 6) < kCols) {                      // uniform over the warp
             uint32_t y[8];
             const uint4* gp = reinterpret_cast<const uint4*>(buf + t * kOutRow + blk * 64 + half * 16);
@@ -598,7 +588,7 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int row = (ep_tid >> 4) + 8 * j;
-            const int n = n0 + c0 + row;
+            const int n = c0 + row;
             if (n < cnt && m < p.M) {
               const long long to = p.row_map ? (long long)p.row_map[row_e + n] : row_e + n;
               if (to >= 0)
@@ -612,7 +602,7 @@ group_mm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           if (m < p.M) {
 #pragma unroll
             for (int i = 0; i < (TILE_N < 32 ? TILE_N : 32); ++i) {
-              const int n = n0 + c0 + i;
+              const int n = c0 + i;
               if (n < cnt) {
                 const long long to = p.row_map ? (long long)p.row_map[row_e + n] : row_e + n;
                 if (to >= 0)

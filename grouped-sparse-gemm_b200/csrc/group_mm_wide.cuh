@@ -1,6 +1,6 @@
 // group_mm, wide token tiles (64 to 256 tokens per tile): prefill-sized problems.
 //
-// Included by group_mm.cu inside namespace pnv::{anonymous}, after Params, TileWalk and the status codes.
+// Included by group_mm.cu inside namespace pnv::{anonymous}, after Params and the status codes.
 //
 // One kernel in two forms.
 //   single CTA (kPair = false)  one CTA per SM multiplies 128 weight rows by TILE_N tokens per tile.
