@@ -215,9 +215,10 @@ __device__ __forceinline__ void tanh_parts(float x, float& num, float& den) {
 }
 
 // SiTU in the form 0.5 (1 + tanh(g / 2)) = 1 / (1 + exp(-g)), everything over one common denominator: three exponentials
-// and one reciprocal where the expression has three tanhf and their divisions.  The approximate exponential and
-// reciprocal are good to a few units in the last place of a float, as tanhf is; for negative gates, where 1 + tanhf(g / 2)
-// cancels, the result is nearer to the exact one.  Not yet rounded to bf16.  (With tanhf the unfused layer of 8192 tokens on
+// and one reciprocal where the expression has three tanhf and their divisions.  For gates of unit size the result is good
+// to 1e-7 before its rounding, as the expression's is; the exponent's product with log2(e) is rounded first, so the error
+// grows with |g| to 5e-6 at 80, far below a bf16 unit; for negative gates, where 1 + tanhf(g / 2) cancels, the result is
+// nearer to the exact one.  Not yet rounded to bf16.  (With tanhf the unfused layer of 8192 tokens on
 // 128 experts of 3072 x 3072 took 1103 us, in this form 969.)
 __device__ __forceinline__ float situ_short(float g, float u, float beta, float inv_beta, float linear_beta, float inv_linear) {
   float gn, gd;
@@ -240,9 +241,9 @@ __device__ __forceinline__ float silu_direct(float g) {
   float s = __fdiv_rn(g, __fadd_rn(1.0f, expf(-g)));
   return __bfloat162float(__float2bfloat16_rn(s));
 }
-// The same bits in a handful of instructions: the approximate exponential and reciprocal are good to a few units in the
-// last place of a float, and for none of the 65536 bf16 gates does that move the result across a bf16 rounding boundary
-// (checked for every pattern by the tests).  The direct form's expf and IEEE division cost about 40 instructions with a
+// The same bits in a handful of instructions: the approximate exponential and reciprocal are good to 1e-7 for gates of unit
+// size and to 5e-6 at |g| = 80 (the exponent's product is rounded), and for none of the 65536 bf16 gates does that move the
+// result across a bf16 rounding boundary (checked for every pattern by the tests).  The direct form's expf and IEEE division cost about 40 instructions with a
 // slow-path branch; a 65536-entry table in global memory cost one gathered load per gate, which the L1 serves at about
 // 14 cycles per warp - that, not memory, was the bound of both users (gated quantizer 57 us for 12000 x 2880 outputs).
 __device__ __forceinline__ float silu_short(float g) {

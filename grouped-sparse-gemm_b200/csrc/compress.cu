@@ -5,12 +5,12 @@
 //           in-chunk indices of the kept bytes, in 128-row x 16-byte atoms (see common.cuh)
 //   sfa     swizzled scale atoms, slop bytes zero
 //
-// Bound: HBM (one layer's 8 x 28672 x 4096 weights: 499 MB in, 323 MB out, 124 us at 6.65 TB/s).  One kernel, a block per
+// Bound: HBM (one layer's 8 x 28672 x 4096 weights: 499 MB in, 323 MB out, 126 us at the measured copy rate of 6.55 TB/s).  One kernel, a block per
 // tile of 128 rows x 1024 K: a lane reads 32 bytes (8 chunks), emits 16 bytes of a_comp and 4 bytes of metadata, a quad of
 // lanes owns one (row, 256-K) metadata line, and a lane has four lines in flight; then a lane per 16-byte line of the
 // tile's scale atoms.  The divisions that place a tile are made once per block, and a chunk costs about 15 instructions
 // without branches.  With per-lane 64-bit divisions, a data-dependent select loop per chunk and byte-sized scale loads in a
-// second kernel these weights took 1166 us, now 122.
+// second kernel these weights took 1166 us, now 128 to 133.
 #include "common.cuh"
 
 namespace pnv {

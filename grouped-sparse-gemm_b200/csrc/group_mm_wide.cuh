@@ -35,7 +35,8 @@
 //            the slot is filled.  In the second CTA of a pair it only relays "my side copies have landed".
 //   4 - 19   epilogue, four groups of four warps (one warp per lane quarter); a tile's chunks of token
 //            columns are dealt round-robin to the groups
-// 20 warps leave 96 registers a thread (five warps to each quarter of the SM); 21 or more leave 80, which spilled.
+// 20 warps leave 96 registers a thread (five warps to each quarter of the SM); 21 or more leave 80, which spilled much more:
+// at 96 the plain 256-token forms spill 12 to 24 bytes a thread, the others nothing.
 //
 // Barriers per pipeline stage s: full[s] (this CTA's copies landed; in a pair's first CTA it also counts the
 // second CTA's tile loads), peer_full[s] (pair: the second CTA's bulk copies landed, relayed to the first), sf_full[s]
@@ -44,7 +45,8 @@
 // warps of the CTA or pair -> issuer).  Every wait is bounded.
 //
 // What bounds it.  A CTA's TMA takes in about 64 bytes per cycle when its requests are 128 bytes wide; a 64-byte
-// request costs as much as a 128-byte one.  Hence 512-K stages (128-byte weight rows) wherever K has more than 256:
+// request costs as much as a 128-byte one.  Hence 512-K stages (128-byte weight rows) in the 256 x 256 pair wherever K has more
+// than 256 (the other variants run the stage depth of their names):
 // 953 cycles per 58 KB stage of the 256 x 256 pair without an epilogue, against 815 per 29 KB with 256-K stages.  Short
 // K loops are bound by the epilogue instead (see there).
 

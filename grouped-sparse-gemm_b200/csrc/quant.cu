@@ -12,8 +12,8 @@
 // Bound: HBM for plain rows (131072 rows of 2048: 118 us, 687 MB), issue slots (0.68 of them used) and L2 for gathered
 // ones (102 us; 150 MB written, the rows read from L2 eight times over), the special-function unit and issue for SiTU.
 // Loads are 32 bytes a lane where the input is aligned to that: 16-byte loads at a stride of 64 bytes take twice the
-// passes through L1.  Before, a warp per 16-byte line of the scale buffer, dead lines included: 466 us for 32768 live
-// rows of 3072 (SiTU) in a capacity of 524288, now 172; the gather of those rows 82 us, now 40.
+// passes through L1.  A warp per 16-byte line of the scale buffer, dead lines included, took 466 us for 32768 live rows of
+// 3072 (SiTU) in a capacity of 524288 where the row form takes 172, and 82 us for the gather of those rows where it takes 40.
 //
 // scatter_quant_act is driven by a flat routing list instead (source token -> destination row), so its scale buffer is
 // pre-filled with a memset node.
@@ -512,7 +512,7 @@ __device__ __forceinline__ void warp_copy(const uint4* __restrict__ src, uint4* 
       if (v0 + i * 32 + lane < n) dst[v0 + i * 32 + lane] = x[i];
   }
 }
-constexpr int kCopyBlocks = 3;      // blocks per SM of the kernels that copy rows (80 registers)
+constexpr int kCopyBlocks = 3;      // blocks per SM of the kernels that copy rows (70 to 80 registers)
 
 // One word of scales: K-blocks 4 kt ... of a row in natural order (`words`: the row can be read by aligned words); blocks
 // past K become the benign byte.

@@ -186,15 +186,15 @@ def test_compress_rejects_per16_scales(ops):
 
 
 def test_silu_table_matches_direct_evaluation(ops):
-    """SiLU goes through a 65536-entry table filled on the device; every possible gate value (all bf16 bit
-    patterns, NaNs and infinities included) must give the same bits as evaluating the expression."""
+    """SiLU is evaluated in a short form (set_silu_table keeps its name from the table that came before it); every possible
+    gate value (all bf16 bit patterns, NaNs and infinities included) must give the same bits as the expression itself."""
     from paired_nvfp4_kernels import ops as pyops
     bits = np.arange(65536, dtype=np.uint16).reshape(2048, 32)
     rng = np.random.default_rng(7)
     for up_scale in (1.0, 37.5):
         up = orc.f32_to_bf16_bits((rng.standard_normal((2048, 32)) * up_scale).astype(np.float32))
         if up_scale == 1.0:
-            up[:] = 0x3F80          # up = 1: the output is the table entry itself
+            up[:] = 0x3F80          # up = 1: the output is the activation itself
         x2 = bf16_tensor(np.concatenate([bits, up], axis=1)[None])
         try:
             y_table = bf16_bits(ops.gated_act(x2))
