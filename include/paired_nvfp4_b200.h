@@ -263,7 +263,9 @@ const char* pnv_group_mm_config_name(int config_id);
  * to the SMs, a tile shared by several CTAs is summed from fp32 partials in K order by whichever arrives
  * last (so the result does not depend on timing).  The first 4 * experts * ceil(features / 128) bytes are
  * arrival counters: they must be zero before the first launch that uses the buffer, every launch leaves
- * them zero, and two launches that may overlap on the GPU must not share a workspace.  Launches with
+ * them zero, and two launches that may overlap on the GPU must not share a workspace.  Nor may launches with another
+ * number of counters, unless the counters are cleared in between: the partial sums follow the counters, so one launch
+ * leaves sums where the other's counters are.  Launches with
  * k < PNV_SPLIT_MIN_K never split, so they need none (a split has to save six K stages of 512). */
 #define PNV_SPLIT_MIN_K 3073
 int64_t pnv_group_mm_workspace_bytes(int experts, int features, int max_n, int sm_count);
